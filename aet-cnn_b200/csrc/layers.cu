@@ -784,13 +784,8 @@ extern "C" int aet_layer_write(aet_layer *l, aet_param which, const void *host_v
     case AET_P_ROLLING_VARIANCE: return write_vec(l, l->rolling_variance, host, l->oc, nullptr);
     case AET_P_MEAN: return write_vec(l, l->mean, host, l->oc, nullptr);
     case AET_P_VARIANCE: return write_vec(l, l->variance, host, l->oc, nullptr);
-    case AET_P_OUTPUT:
-        l->output->lazy_zero = false;
-        l->output_stale = false;
-        l->lin_out_stale = false;
-        return aet_tensor_write(l->output, host);
+    case AET_P_OUTPUT: return aet_tensor_write(l->output, host);
     case AET_P_DELTA:
-        l->delta->lazy_zero = false;
         l->lin_delta_stale = false;
         l->stem_delta_stale = false;
         return aet_tensor_write(l->delta, host);

@@ -898,10 +898,17 @@ extern "C" int aet_tensor_shape(const aet_tensor *t, int *batch, int *c, int *h,
     return AET_OK;
 }
 extern "C" size_t aet_tensor_count(const aet_tensor *t) { return t ? t->count() : 0; }
+// The caller's values replace whatever the tensor was still to be filled with.
+static void tensor_overwritten(aet_tensor *t) {
+    t->touched = true;
+    if (t->owner) t->owner->output_stale = t->owner->lin_out_stale = false;
+}
+
 extern "C" int aet_tensor_write(aet_tensor *t, const float *host_nchw) {
     ctx_enter(t ? t->ctx : nullptr);
     if (!t || !host_nchw) { aet_set_error("aet_tensor_write: null argument"); return AET_E_INVALID; }
-    t->touched = true;
+    tensor_overwritten(t);
+    t->lazy_zero = false;
     return tensor_upload_nchw(t->ctx, t->d, host_nchw, t->n, t->c, t->h, t->w, t->cp);
 }
 extern "C" int aet_tensor_read(const aet_tensor *t, float *host_nchw) {
@@ -913,7 +920,7 @@ extern "C" int aet_tensor_read(const aet_tensor *t, float *host_nchw) {
 extern "C" int aet_tensor_zero(aet_tensor *t) {
     ctx_enter(t ? t->ctx : nullptr);
     if (!t) { aet_set_error("null tensor"); return AET_E_INVALID; }
-    t->touched = true;
+    tensor_overwritten(t);
     AET_CUDA(cudaMemsetAsync(t->d, 0, t->elems() * sizeof(float), t->ctx->stream));
     return AET_OK;
 }

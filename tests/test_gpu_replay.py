@@ -1,0 +1,41 @@
+"""What calls leave behind and find: replayed passes, outputs that a fused pass left out, streams that cannot be captured."""
+import os
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def cifar(aet, ctx, batch=8, train=1):
+    return aet.NNetwork(ctx, cfg_path=os.path.join(aet.CFG_DIR, "cifar_small.cfg"), train=train, batch=batch)
+
+
+def batches(net, count, seed=11):
+    rng = np.random.default_rng(seed)
+    for _ in range(count):
+        x = rng.random(net.input_shape, dtype=np.float32)
+        t = np.eye(net.outputs, dtype=np.float32)[rng.integers(0, net.outputs, net.batch)]
+        yield x, t
+
+
+@pytest.mark.parametrize("replayed", [False, True])
+def test_written_output_is_kept(aet, ctx, replayed):
+    """What a program writes into an output tensor replaces what a fused pass left to be formed there."""
+    net = cifar(aet, ctx)
+    net.use_graph(replayed)
+    head = net.layer_count - 3
+    for x, t in batches(net, 3):
+        net.train(x, t)
+    for i in (0, head):
+        out = net.layer(i).output
+        v = np.random.default_rng(i).standard_normal(out.shape).astype(np.float32)
+        for k in range(3):
+            net.predict(x) if k else net.train(x, t)
+            out.write(v)
+            assert np.array_equal(out.read(), v), (i, k)
+            assert np.array_equal(net.layer(i).read(aet.P_OUTPUT), v.ravel()), (i, k)
+            net.predict(x) if k else net.train(x, t)
+            out.zero()
+            assert not out.read().any(), (i, k)
+    net.close()
