@@ -417,18 +417,21 @@ void flags_save(const aet_network *net, std::vector<LayerFlags> &out) {
         out.push_back(f);
     }
 }
-void flags_restore(aet_network *net, const std::vector<LayerFlags> &in) {
+// A prediction (`backward` = false) leaves what belongs to the deltas as it finds it, as the plain pass does.
+void flags_restore(aet_network *net, const std::vector<LayerFlags> &in, bool backward) {
     for (size_t i = 0; i < in.size(); ++i) {
         aet_layer *l = net->layers[i];
         const LayerFlags &f = in[i];
         if (l->output) l->output->lazy_zero = f.output_zero;
-        if (l->delta) l->delta->lazy_zero = f.delta_zero;
         l->output_stale = f.output_stale; l->last_forward_train = f.last_forward_train; l->fused_ready = f.fused_ready;
-        l->gather_pending = f.gather_pending; l->lin_fwd_pending = f.lin_fwd_pending; l->lin_used = f.lin_used;
+        l->lin_fwd_pending = f.lin_fwd_pending; l->lin_used = f.lin_used;
         l->lin_out_stale = f.lin_out_stale; l->lin_bwd_pending = f.lin_bwd_pending; l->lin_delta_stale = f.lin_delta_stale;
-        l->head_forward_pending = f.head_forward_pending; l->head_backward_done = f.head_backward_done;
+        l->head_forward_pending = f.head_forward_pending;
         l->stem_gram_ready = f.stem_gram_ready; l->stem_delta_stale = f.stem_delta_stale;
         l->lin_input = f.lin_input; l->s2d_src = f.s2d_src;
+        if (!backward) continue;
+        if (l->delta) l->delta->lazy_zero = f.delta_zero;
+        l->gather_pending = f.gather_pending; l->head_backward_done = f.head_backward_done;
     }
 }
 
@@ -437,7 +440,7 @@ void flags_restore(aet_network *net, const std::vector<LayerFlags> &in) {
 // capturing and instantiating takes about a millisecond), unless the caller's stream is being captured itself, the
 // launches are being profiled, or graphs are switched off (first_capture < 0).
 template <typename Body>
-int run_pass(aet_network *net, PassGraph &g, EagerRuns &eager, int first_capture, Body body) {
+int run_pass(aet_network *net, PassGraph &g, EagerRuns &eager, int first_capture, bool backward, Body body) {
     aet_context *ctx = net->ctx;
     if (g.exec && g.epoch != ctx->epoch) graph_release(g);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -447,7 +450,7 @@ int run_pass(aet_network *net, PassGraph &g, EagerRuns &eager, int first_capture
     if (graphs && g.exec) {
         AET_CUDA(cudaGraphLaunch(g.exec, ctx->stream));
         ctx->launches += g.launches;
-        flags_restore(net, g.flags);
+        flags_restore(net, g.flags, backward);
         return AET_OK;
     }
     const long before = ctx->launches;
@@ -906,7 +909,7 @@ extern "C" int aet_network_train_step_device(aet_network *net, float *loss) {
     if (g.exec && net->graph_clean[gi] != clean_now) graph_release(g);   // captured in the other arena state
     net->graph_clean[gi] = clean_now;
     const int first_capture = net->use_graph == 1 ? 1 : (net->use_graph == 2 && !net->comm ? 8 : -1);
-    AET_TRY(run_pass(net, g, net->eager[kind], first_capture, [&] { return run_step(net, final); }));
+    AET_TRY(run_pass(net, g, net->eager[kind], first_capture, true, [&] { return run_step(net, final); }));
     net->grad_clean = final;
     if (final) net->launches_per_step = ctx->launches - before;
     if (loss) return aet_network_last_loss(net, loss);
@@ -1113,7 +1116,7 @@ int slot_run(aet_network *net, PredictSlot &s, int mode, int k) {
     if (mode == 1 && s.k != k) { graph_release(s.graph[1]); s.k = k; }
     net->input->touched = true;
     const int first_capture = net->use_graph ? 1 : -1;
-    return run_pass(net, s.graph[mode], net->predict_eager[mode], first_capture, [&]() -> int {
+    return run_pass(net, s.graph[mode], net->predict_eager[mode], first_capture, false, [&]() -> int {
         aet_tensor *in = s.in;
         pdl_skip_next();   // behind copies, or the first node of a graph
         if (in->count() * sizeof(float) <= kDirectBytes)

@@ -39,3 +39,25 @@ def test_written_output_is_kept(aet, ctx, replayed):
             out.zero()
             assert not out.read().any(), (i, k)
     net.close()
+
+
+def test_replayed_prediction_leaves_the_deltas(aet, ctx):
+    """A prediction captured while the deltas counted as cleared does not clear them when it is replayed later."""
+    out = []
+    for graph in (True, False):
+        net = cifar(aet, ctx)
+        net.use_graph(graph)
+        (x, t), = batches(net, 1)
+        net.input.write(x)
+        net.truth.write(t)
+        st = aet.make_state(input=net.input, truth=net.truth, train=1)
+        net.forward(st)
+        for _ in range(3):
+            net.predict(x)
+        net.forward(st)
+        net.backward(st)
+        net.predict(x)
+        out.append([net.layer(i).read(aet.P_DELTA) for i in range(1, net.layer_count - 3)])
+        net.close()
+    for a, b in zip(*out):
+        assert b.any() and np.array_equal(a, b)
