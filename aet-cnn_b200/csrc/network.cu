@@ -432,6 +432,7 @@ void flags_restore(aet_network *net, const std::vector<LayerFlags> &in, bool bac
         if (!backward) continue;
         if (l->delta) l->delta->lazy_zero = f.delta_zero;
         l->gather_pending = f.gather_pending; l->head_backward_done = f.head_backward_done;
+        l->cost_valid = false;   // every softmax layer of the pass has a new cost
     }
 }
 

@@ -61,3 +61,36 @@ def test_replayed_prediction_leaves_the_deltas(aet, ctx):
         net.close()
     for a, b in zip(*out):
         assert b.any() and np.array_equal(a, b)
+
+
+SOFTMAXES_CFG = """[net]
+batch=4
+width=1
+height=1
+channels=10
+learning_rate=0.5
+[convolutional]
+filters=10
+size=1
+activation=linear
+[softmax]
+[convolutional]
+filters=10
+size=1
+activation=linear
+[softmax]
+"""
+
+
+def test_cost_of_every_softmax_after_replayed_steps(aet, ctx):
+    out = []
+    for graph in (True, False):
+        net = aet.NNetwork(ctx, cfg_text=SOFTMAXES_CFG, train=1)
+        net.use_graph(graph)
+        got = []
+        for x, t in batches(net, 6):
+            net.train(x, t)
+            got.append(net.cost())
+        out.append(got)
+        net.close()
+    assert out[0] == out[1]
