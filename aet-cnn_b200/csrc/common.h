@@ -154,6 +154,7 @@ struct aet_tensor {
     // accumulating, and host reads return zeros.  Lets the network skip one memset per layer.
     bool lazy_zero = false;
     aet_layer *owner = nullptr;   // a convolution's output: a fused pass may leave it to be formed when somebody reads it
+    aet_layer *reader = nullptr;  // a linear head's convolution: it forms its left-out output from this tensor
     bool touched = false;   // written outside the training step since the pipelined step last looked (network inputs)
     size_t count() const { return (size_t)n * c * h * w; }
     size_t elems() const { return (size_t)n * h * w * cp; }  // device floats
@@ -478,6 +479,8 @@ int side_begin(aet_context *ctx);
 void side_end(aet_context *ctx);
 int side_join(aet_context *ctx);
 int layer_form_output(aet_layer *l);   // forms an output tensor that a fused pass left out
+int layer_settle_prediction(aet_layer *l);
+int tensor_settle(const aet_tensor *t);      // before `t` changes: forms what is still to be formed from it
 // Entry points make their context's device the calling thread's current one: a process may hold contexts on several
 // GPUs (or another library may have switched the device), and allocations and launches follow the current device.
 static inline void ctx_enter(const aet_context *ctx) {

@@ -331,6 +331,13 @@ int layer_form_output(aet_layer *l) {
     return AET_OK;
 }
 
+// Before an update: a prediction's output is formed with the prediction's weights.  (A training pass is followed by its own
+// update: forming the output there would cost each step the convolution that the head saves.)
+int layer_settle_prediction(aet_layer *l) { return l->lin_out_stale && !l->lin_used ? layer_form_output(l) : AET_OK; }
+int tensor_settle(const aet_tensor *t) {
+    return t->reader && t->reader->lin_out_stale ? layer_form_output(t->reader) : AET_OK;
+}
+
 static int check_input(const aet_layer *l, const aet_tensor *in) {
     if (!in) return fail_invalid("layer forward/backward: state.input is NULL");
     if (in->n != l->batch || in->c != l->c || in->h != l->h || in->w != l->w) {
@@ -362,6 +369,10 @@ extern "C" int aet_layer_forward(aet_layer *l, aet_state state) {
     l->ctx->prof_tag = l->net ? l->index : -1;
     AET_TRY(check_input(l, state.input));
     if (state.input->owner && state.input->owner->lin_out_stale) AET_TRY(layer_form_output(state.input->owner));   // an input from another pass
+    if (!l->ctx->in_network_pass) {   // a network's pass renews what is formed from its outputs
+        AET_TRY(tensor_settle(l->output));
+        if (l->fused_pool) AET_TRY(tensor_settle(l->fused_pool->output));
+    }
     switch (l->type) {
     case AET_CONVOLUTIONAL:
         if (l->bn) {
@@ -389,8 +400,9 @@ extern "C" int aet_layer_forward(aet_layer *l, aet_state state) {
             }
         } else {
             l->lin_used = false; l->lin_out_stale = false; l->lin_delta_stale = false; l->lin_bwd_pending = false;
-            if (l->lin_head && l->ctx->in_network_pass && (!state.train || state.truth)) {
-                // classifier head of a network: folded into the softmax layer's call
+            if (l->lin_head && l->ctx->in_network_pass && (state.train ? state.truth != nullptr : l->index > 0)) {
+                // classifier head of a network: folded into the softmax layer's call.  (A prediction's output has to stay
+                // what it was until somebody reads it: where the input is the caller's tensor, nothing here sees that change.)
                 l->lin_fwd_pending = true;
                 l->lin_input = state.input;
                 l->output->lazy_zero = false;
@@ -604,6 +616,7 @@ extern "C" int aet_layer_update(aet_layer *l, int batch, float learning_rate, fl
     // CPU update does not (dnn/ConvolutionalLayer.c:959-980)
     const int scrub_w = l->ctx->parity == AET_PARITY_MTCS ? 1 : 0;
     const int scrub_bn = (l->bn && l->net && l->net->try_fix_nan && l->ctx->parity == AET_PARITY_MTCS) ? 2 : 0;
+    AET_TRY(layer_settle_prediction(l));
     AET_TRY(k_sgd_segment(l->ctx, layer_W(l), layer_U(l), layer_G(l), l->seg_w.padded, rate, momentum, -decay * batch * loss_scale, scrub_w));
     AET_TRY(k_sgd_segment(l->ctx, layer_b(l), layer_bU(l), layer_bG(l), l->seg_b.padded, rate, momentum, 0.f, scrub_bn));
     if (l->bn) AET_TRY(k_sgd_segment(l->ctx, layer_s(l), layer_sU(l), layer_sG(l), l->seg_s.padded, rate, momentum, 0.f, scrub_bn));
@@ -769,6 +782,7 @@ extern "C" int aet_layer_write(aet_layer *l, aet_param which, const void *host_v
     if (aet_layer_param_count(l, which) == 0) return fail_invalid("aet_layer_write: this layer has no such buffer");
     const float *host = static_cast<const float *>(host_v);
     aet_context *ctx = l->ctx;
+    if (l->lin_out_stale && (which == AET_P_WEIGHTS || which == AET_P_BIASES)) AET_TRY(layer_form_output(l));
     switch (which) {
     case AET_P_WEIGHTS:
         return tensor_upload_nchw(ctx, layer_W(l), host, l->oc, l->cg, l->size, l->size, l->cgp);

@@ -714,8 +714,10 @@ extern "C" aet_network *aet_network_create_ex(aet_context *ctx, const char *cfg_
                     (size_t)(cv->batch + 256) * l->c * sizeof(float) <= 40 * 1024 && (size_t)(cv->cp + 32) * sizeof(float) <= 40 * 1024 &&
                     cudaMalloc(&cv->lin_xbar, (size_t)cv->batch * cv->cp * sizeof(float)) == cudaSuccess &&
                     cudaMalloc(&cv->lin_ticket, sizeof(unsigned int)) == cudaSuccess &&
-                    cudaMemset(cv->lin_ticket, 0, sizeof(unsigned int)) == cudaSuccess)
+                    cudaMemset(cv->lin_ticket, 0, sizeof(unsigned int)) == cudaSuccess) {
                     cv->lin_head = true;
+                    if (cv->index > 0) net->layers[cv->index - 1]->output->reader = cv;
+                }
             }
         }
         c = l->oc; h = l->oh; w = l->ow;
@@ -863,6 +865,7 @@ extern "C" int aet_network_backward(aet_network *net, aet_state state) {
 extern "C" int aet_network_update(aet_network *net) {
     ctx_enter(net ? net->ctx : nullptr);
     if (!net) { aet_set_error("null network"); return AET_E_INVALID; }
+    for (aet_layer *l : net->layers) AET_TRY(layer_settle_prediction(l));
     AET_TRY(upload_hyper(net));
     net->ctx->prof_tag = -1;   // the update belongs to no single layer
     if (net->n_blocks) AET_TRY(net->adam ? k_adam_arena(net) : k_sgd_arena(net));

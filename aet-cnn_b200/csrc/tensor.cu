@@ -907,6 +907,7 @@ static void tensor_overwritten(aet_tensor *t) {
 extern "C" int aet_tensor_write(aet_tensor *t, const float *host_nchw) {
     ctx_enter(t ? t->ctx : nullptr);
     if (!t || !host_nchw) { aet_set_error("aet_tensor_write: null argument"); return AET_E_INVALID; }
+    AET_TRY(tensor_settle(t));
     tensor_overwritten(t);
     t->lazy_zero = false;
     return tensor_upload_nchw(t->ctx, t->d, host_nchw, t->n, t->c, t->h, t->w, t->cp);
@@ -920,6 +921,7 @@ extern "C" int aet_tensor_read(const aet_tensor *t, float *host_nchw) {
 extern "C" int aet_tensor_zero(aet_tensor *t) {
     ctx_enter(t ? t->ctx : nullptr);
     if (!t) { aet_set_error("null tensor"); return AET_E_INVALID; }
+    AET_TRY(tensor_settle(t));
     tensor_overwritten(t);
     AET_CUDA(cudaMemsetAsync(t->d, 0, t->elems() * sizeof(float), t->ctx->stream));
     return AET_OK;

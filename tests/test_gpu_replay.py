@@ -4,6 +4,9 @@ import os
 import numpy as np
 import pytest
 
+from conftest import rel_l2
+from gpu_util import TOL_TF32
+
 pytestmark = pytest.mark.gpu
 
 
@@ -94,3 +97,41 @@ def test_cost_of_every_softmax_after_replayed_steps(aet, ctx):
         out.append(got)
         net.close()
     assert out[0] == out[1]
+
+
+def test_left_out_head_output_is_the_one_of_its_pass(aet, ctx, tmp_path):
+    """The classifier convolution's output, which a prediction leaves out, is that of the prediction's weights and input,
+    whatever is written before it is read."""
+    net = cifar(aet, ctx)
+    ctx.set_option("linear_head", 0)
+    try:
+        plain = cifar(aet, ctx)
+    finally:
+        ctx.set_option("linear_head", 1)
+    (x, t), = batches(net, 1)
+    net.save_weights(str(tmp_path / "w"))
+    plain.load_weights(str(tmp_path / "w"))
+    plain.predict(x)
+    at = net.layer_count - 3
+    want = plain.layer(at).read(aet.P_OUTPUT)
+    head, before = net.layer(at), net.layer(at - 1)
+    w, b = head.read(aet.P_WEIGHTS), head.read(aet.P_BIASES)
+
+    def by_hand():
+        st = aet.make_state(input=net.layer(at - 2).output, train=0)
+        net.layer(at - 2).output.write(np.zeros(net.layer(at - 2).output.shape, np.float32))
+        before.forward(st)
+
+    changes = [lambda: head.write(aet.P_WEIGHTS, 2 * w), lambda: head.write(aet.P_BIASES, b + 1),
+               lambda: before.output.write(np.ones(before.output.shape, np.float32)), lambda: before.output.zero(), by_hand, net.update,
+               lambda: head.update(net.batch, 0.1, 0.9, 0.1)]
+    for replayed in (False, True):
+        net.use_graph(replayed)
+        for n, change in enumerate(changes):
+            net.load_weights(str(tmp_path / "w"))
+            for _ in range(3):
+                net.predict(x)
+            change()
+            assert rel_l2(head.read(aet.P_OUTPUT), want) <= TOL_TF32, (replayed, n)
+    net.close()
+    plain.close()
