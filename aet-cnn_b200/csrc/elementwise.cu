@@ -2420,7 +2420,7 @@ int k_augment(aet_context *ctx, const float *src_nchw, int n, int c, int sh, int
 
 int k_top_k(aet_context *ctx, const float *scores, int samples, int n, int ld, int k, int *index_dev) {
     LaunchScope s(ctx, "top_k", 4.0 * samples * n, 0);
-    if (k <= 32)
+    if (k <= kTopkLanes)
         launch_k(ctx->stream, (unsigned)((samples + TOPK_WARPS - 1) / TOPK_WARPS), TOPK_WARPS * 32, 0, top_k_warp_kernel, scores, samples, n, ld,
                  k, index_dev);
     else

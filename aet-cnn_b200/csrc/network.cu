@@ -1119,6 +1119,8 @@ int slot_run(aet_network *net, PredictSlot &s, int mode, int k) {
     aet_context *ctx = net->ctx;
     if (mode == 1 && s.k != k) { graph_release(s.graph[1]); s.k = k; }
     net->input->touched = true;
+    float *list = nullptr;   // the long lists are worked on in memory, not across the link (sized here: a capture cannot allocate)
+    if (mode == 1 && k > kTopkLanes) AET_TRY(ctx_scratch(ctx, predict_out_bytes(net, 1, k), &list));
     const int first_capture = net->use_graph ? 1 : -1;
     return run_pass(net, s.graph[mode], net->predict_eager[mode], first_capture, false, [&]() -> int {
         aet_tensor *in = s.in;
@@ -1132,11 +1134,10 @@ int slot_run(aet_network *net, PredictSlot &s, int mode, int k) {
         const aet_layer *last = net->layers.back();
         void *out = s.pin + kSlotOut;
         if (mode == 0) return tensor_download_staged(ctx, last->output->d, static_cast<float *>(out), last->batch, last->oc, last->oh, last->ow, last->ocp);
-        if (k <= 32) return k_top_k(ctx, last->output->d, net->batch, last->oc, last->ocp, k, static_cast<int *>(out));
-        float *scratch = nullptr;   // the long lists are worked on in memory: not across the link
-        AET_TRY(ctx_scratch(ctx, (size_t)net->batch * k * sizeof(int), &scratch));
-        AET_TRY(k_top_k(ctx, last->output->d, net->batch, last->oc, last->ocp, k, reinterpret_cast<int *>(scratch)));
-        AET_CUDA(cudaMemcpyAsync(out, scratch, (size_t)net->batch * k * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        if (k <= kTopkLanes) return k_top_k(ctx, last->output->d, net->batch, last->oc, last->ocp, k, static_cast<int *>(out));
+        AET_TRY(ctx_scratch(ctx, predict_out_bytes(net, 1, k), &list));   // the forward pass may have moved it
+        AET_TRY(k_top_k(ctx, last->output->d, net->batch, last->oc, last->ocp, k, reinterpret_cast<int *>(list)));
+        AET_CUDA(cudaMemcpyAsync(out, list, predict_out_bytes(net, 1, k), cudaMemcpyDeviceToHost, ctx->stream));
         return AET_OK;
     });
 }

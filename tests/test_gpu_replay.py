@@ -135,3 +135,36 @@ def test_left_out_head_output_is_the_one_of_its_pass(aet, ctx, tmp_path):
             assert rel_l2(head.read(aet.P_OUTPUT), want) <= TOL_TF32, (replayed, n)
     net.close()
     plain.close()
+
+
+TOPK_CFG = """[net]
+batch=4
+width=1
+height=1
+channels=8
+learning_rate=0.01
+[convolutional]
+filters=%d
+size=1
+activation=linear
+[softmax]
+"""
+
+
+def test_top_k_list_grows_between_calls(aet, oracle):
+    """A context of its own, so that nothing else has sized its scratch memory."""
+    ctx = aet.Context(0)
+    classes = 60
+    net = aet.NNetwork(ctx, cfg_text=TOPK_CFG % classes, train=0)
+    rng = np.random.default_rng(5)
+    net.layer(0).write(aet.P_WEIGHTS, rng.standard_normal((classes, 8, 1, 1)).astype(np.float32))
+    x = rng.random((4, 8, 1, 1), dtype=np.float32)
+    ids = np.arange(4, dtype=np.int32)
+    for k in (5, 40, 40, 40, 5, 60, 60, 5, 40):
+        idx = net.predict_topk(x, k)
+        net.validate(x, ids, k)
+        score = net.predict(x).reshape(4, classes)
+        for i in range(4):
+            assert np.array_equal(idx[i], oracle.top_k(score[i], k)), (k, i)
+    net.close()
+    ctx.close()
