@@ -100,6 +100,7 @@ struct aet_context {
     int sm_count = 148;
     cudaStream_t stream = nullptr;
     bool owns_stream = false;
+    bool stream_apart = true;   // the stream does not synchronise with the legacy default stream
     aet_parity_mode parity = AET_PARITY_MTCS;
     aet_math_mode math = AET_MATH_TF32;
     int conv_path = 0;  // 0 auto (TMA where the shape allows), 1 force gather producer
@@ -290,7 +291,7 @@ struct PassGraph {
 // Eager passes of one kind since the context's epoch changed last: the first one sizes the scratch buffers, and only a
 // pass that has run before is worth capturing.
 struct EagerRuns {
-    unsigned long long epoch = 0;
+    unsigned long long epoch = 0, refused = 0;   // refused: the context's epoch at which a capture failed
     int count = 0;
 };
 // Buffers of one prediction in flight: the input tensor (slot 0: the network's), a page-locked block (images on their way

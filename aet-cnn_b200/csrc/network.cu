@@ -436,16 +436,42 @@ void flags_restore(aet_network *net, const std::vector<LayerFlags> &in, bool bac
     }
 }
 
+// Captures the pass, instantiates its graph and launches that.  After an error nothing of the pass has run.
+template <typename Body>
+int capture_pass(aet_network *net, PassGraph &g, Body body) {
+    aet_context *ctx = net->ctx;
+    const long before = ctx->launches;
+    cudaGraph_t graph = nullptr;
+    AET_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+    ctx->capturing = true;
+    const int r = body();
+    ctx->capturing = false;
+    cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
+    if (r != AET_OK) { if (graph) cudaGraphDestroy(graph); return r; }
+    if (e != cudaSuccess) { aet_set_error("graph capture failed: %s", cudaGetErrorString(e)); return AET_E_CUDA; }
+    g.launches = ctx->launches - before;
+    g.epoch = ctx->epoch;
+    flags_save(net, g.flags);
+    e = cudaGraphInstantiate(&g.exec, graph, 0);
+    cudaGraphDestroy(graph);
+    if (e != cudaSuccess) { aet_set_error("graph instantiate failed: %s", cudaGetErrorString(e)); g.exec = nullptr; return AET_E_CUDA; }
+    AET_CUDA(cudaGraphLaunch(g.exec, ctx->stream));
+    return AET_OK;
+}
+
 // Runs one pass of launches: replays its graph, captures it, or launches it eagerly.  A launch costs the host 3.4 us and
 // a replay 1 us for the whole pass, so a pass that comes again is captured (`first_capture` eager runs of its kind before;
 // capturing and instantiating takes about a millisecond), unless the caller's stream is being captured itself, the
 // launches are being profiled, or graphs are switched off (first_capture < 0).
+// `asked`: the caller has asked for the graph, so that a capture that fails is the call's error.  Otherwise the pass runs
+// eagerly then, and from then on; and a stream that synchronises with the legacy default stream is left alone, because
+// while it is being captured no other thread could use that one.
 template <typename Body>
-int run_pass(aet_network *net, PassGraph &g, EagerRuns &eager, int first_capture, bool backward, Body body) {
+int run_pass(aet_network *net, PassGraph &g, EagerRuns &eager, int first_capture, bool asked, bool backward, Body body) {
     aet_context *ctx = net->ctx;
     if (g.exec && g.epoch != ctx->epoch) graph_release(g);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    bool graphs = first_capture >= 0 && !ctx->profiling;
+    bool graphs = first_capture >= 0 && !ctx->profiling && (asked || (ctx->stream_apart && eager.refused != ctx->epoch));
     if (graphs && cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess) { cudaGetLastError(); graphs = false; }
     graphs = graphs && cap == cudaStreamCaptureStatusNone;
     if (graphs && g.exec) {
@@ -454,24 +480,16 @@ int run_pass(aet_network *net, PassGraph &g, EagerRuns &eager, int first_capture
         flags_restore(net, g.flags, backward);
         return AET_OK;
     }
-    const long before = ctx->launches;
     if (graphs && eager.epoch == ctx->epoch && eager.count >= first_capture) {
-        cudaGraph_t graph = nullptr;
-        AET_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-        ctx->capturing = true;
-        const int r = body();
-        ctx->capturing = false;
-        cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
-        if (r != AET_OK) { if (graph) cudaGraphDestroy(graph); return r; }
-        if (e != cudaSuccess) { aet_set_error("graph capture failed: %s", cudaGetErrorString(e)); return AET_E_CUDA; }
-        g.launches = ctx->launches - before;
-        g.epoch = ctx->epoch;
-        flags_save(net, g.flags);
-        e = cudaGraphInstantiate(&g.exec, graph, 0);
-        cudaGraphDestroy(graph);
-        if (e != cudaSuccess) { aet_set_error("graph instantiate failed: %s", cudaGetErrorString(e)); g.exec = nullptr; return AET_E_CUDA; }
-        AET_CUDA(cudaGraphLaunch(g.exec, ctx->stream));
-        return AET_OK;
+        const long before = ctx->launches;
+        const bool clean = net->grad_clean;
+        const int r = capture_pass(net, g, body);
+        if (r == AET_OK || asked) return r;
+        cudaGetLastError();
+        graph_release(g);
+        eager.refused = ctx->epoch;
+        ctx->launches = before;
+        net->grad_clean = clean;
     }
     AET_TRY(body());
     if (eager.epoch != ctx->epoch) { eager.epoch = ctx->epoch; eager.count = 0; }
@@ -913,7 +931,7 @@ extern "C" int aet_network_train_step_device(aet_network *net, float *loss) {
     if (g.exec && net->graph_clean[gi] != clean_now) graph_release(g);   // captured in the other arena state
     net->graph_clean[gi] = clean_now;
     const int first_capture = net->use_graph == 1 ? 1 : (net->use_graph == 2 && !net->comm ? 8 : -1);
-    AET_TRY(run_pass(net, g, net->eager[kind], first_capture, true, [&] { return run_step(net, final); }));
+    AET_TRY(run_pass(net, g, net->eager[kind], first_capture, net->use_graph == 1, true, [&] { return run_step(net, final); }));
     net->grad_clean = final;
     if (final) net->launches_per_step = ctx->launches - before;
     if (loss) return aet_network_last_loss(net, loss);
@@ -1122,7 +1140,7 @@ int slot_run(aet_network *net, PredictSlot &s, int mode, int k) {
     float *list = nullptr;   // the long lists are worked on in memory, not across the link (sized here: a capture cannot allocate)
     if (mode == 1 && k > kTopkLanes) AET_TRY(ctx_scratch(ctx, predict_out_bytes(net, 1, k), &list));
     const int first_capture = net->use_graph ? 1 : -1;
-    return run_pass(net, s.graph[mode], net->predict_eager[mode], first_capture, false, [&]() -> int {
+    return run_pass(net, s.graph[mode], net->predict_eager[mode], first_capture, false, false, [&]() -> int {
         aet_tensor *in = s.in;
         pdl_skip_next();   // behind copies, or the first node of a graph
         if (in->count() * sizeof(float) <= kDirectBytes)

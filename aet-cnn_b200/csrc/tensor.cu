@@ -634,6 +634,9 @@ extern "C" int aet_context_set_stream(aet_context *ctx, void *cuda_stream) {
         AET_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
         ctx->owns_stream = true;
     }
+    unsigned int flags = 0;
+    if (cudaStreamGetFlags(ctx->stream, &flags) != cudaSuccess) { cudaGetLastError(); flags = 0; }
+    ctx->stream_apart = (flags & cudaStreamNonBlocking) != 0;
     return AET_OK;
 }
 extern "C" void *aet_context_stream(aet_context *ctx) { return ctx ? (void *)ctx->stream : nullptr; }

@@ -1,5 +1,7 @@
 """What calls leave behind and find: replayed passes, outputs that a fused pass left out, streams that cannot be captured."""
+import ctypes
 import os
+import threading
 
 import numpy as np
 import pytest
@@ -168,3 +170,58 @@ def test_top_k_list_grows_between_calls(aet, oracle):
             assert np.array_equal(idx[i], oracle.top_k(score[i], k)), (k, i)
     net.close()
     ctx.close()
+
+
+def test_legacy_default_stream(aet):
+    """The legacy default stream (handle 1) cannot be captured: predictions and training steps go on as plain launches."""
+    out = []
+    for stream in (1, None):
+        ctx = aet.Context(0, stream=stream)
+        net = cifar(aet, ctx)
+        if stream is None:
+            net.use_graph(False)
+        got = []
+        for x, t in batches(net, 12):
+            got.append(net.train(x, t))
+            got += [net.predict(x).copy(), net.predict_topk(x, 3).copy()]
+        got.append(net.layer(0).read(aet.P_WEIGHTS))
+        out.append(got)
+        net.close()
+        ctx.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
+
+
+def test_blocking_stream_is_not_captured_unasked(aet):
+    """While a stream that synchronises with the legacy default stream is captured, no other thread may use that one."""
+    import torch
+    handle = ctypes.c_void_p()
+    torch.cuda.init()
+    assert int(torch.cuda.cudart().cudaStreamCreate(ctypes.addressof(handle))) == 0
+    ctx = aet.Context(0, stream=handle.value)
+    net = cifar(aet, ctx, batch=2, train=0)
+    x, _ = next(batches(net, 1))
+    want = net.predict_topk(x, 4).copy()
+    stop, failed = threading.Event(), []
+
+    def other():
+        a = torch.zeros(64, device="cuda")
+        try:
+            while not stop.is_set():
+                a.add_(1.0)
+        except RuntimeError as e:
+            failed.append(e)
+
+    worker = threading.Thread(target=other)
+    worker.start()
+    try:
+        for i in range(300):   # a new k is a new pass
+            k = 1 + i // 3 % 4
+            assert np.array_equal(net.predict_topk(x, k), want[:, :k])
+    finally:
+        stop.set()
+        worker.join()
+        net.close()
+        ctx.close()
+        torch.cuda.synchronize()
+        torch.cuda.cudart().cudaStreamDestroy(handle.value)
+    assert not failed, failed
