@@ -175,9 +175,18 @@ conv_igemm_kernel(const __grid_constant__ IgemmMaps maps, const IgemmArgs a) {
     if (warp < 4) {
         // ------------------------------------------------------------------ epilogue
         float *mine = staging + (size_t)(warp * 32) * PITCH;
+        const size_t rows32 = (size_t)prank * 4 + warp;
+        // Lane 0: this warp's place among the parts of its rows, the last one clears the ticket for the next launch.  A warp
+        // whose wait ran out takes its tickets all the same: a part that did not would leave the next launch miscounting.
+        auto take_ticket = [&](int split) {
+            unsigned int *ticket = a.tickets + (size_t)split * (PAIR ? 8 : 4) + rows32;
+            const unsigned int order = atomicAdd(ticket, 1u);
+            if (order == (unsigned)a.parts - 1u) *ticket = 0u;
+            return order;
+        };
         uint32_t tcount = 0;
         bool ok = true;
-        for (int t = unit; t < total_tiles && ok; t += units, ++tcount) {
+        for (int t = unit; t < total_tiles; t += units, ++tcount) {
             const IgemmTile tile = igemm_tile(a, t);
             const IgemmClass &cl = a.cls[tile.cls];
             // this lane's row of the tile, and the output pixel it belongs to (-1: past the end)
@@ -196,9 +205,12 @@ conv_igemm_kernel(const __grid_constant__ IgemmMaps maps, const IgemmArgs a) {
                 }
             }
             const uint32_t b = tcount & 1u;
-            ok = mbar_wait(smem_u32(&ctl.acc_full[b]), (tcount >> 1) & 1u, abort_flag);
+            ok = ok && mbar_wait(smem_u32(&ctl.acc_full[b]), (tcount >> 1) & 1u, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
+            if (!ok) {
+                if (tile.split >= 0 && lane == 0) take_ticket(tile.split);
+                continue;
+            }
             tc_fence_after_sync();
             const bool have = tile.slabs > 0;
             const uint32_t acc = tmem + b * (uint32_t)a.bn + ((uint32_t)(warp * 32) << 16);
@@ -206,7 +218,6 @@ conv_igemm_kernel(const __grid_constant__ IgemmMaps maps, const IgemmArgs a) {
             const float *parts = nullptr;              // this warp's rows of part 0: [column][lane]
             const size_t part_stride = (size_t)a.bn * BM * (PAIR ? 2 : 1);
             if (split) {
-                const size_t rows32 = (size_t)prank * 4 + warp;
                 float *base = a.partial + (size_t)tile.split * a.parts * part_stride + rows32 * 32 * a.bn + lane;
                 float *mine_part = base + (size_t)tile.part * part_stride;
                 for (int c = 0; c < a.bn; c += 16) {
@@ -228,9 +239,7 @@ conv_igemm_kernel(const __grid_constant__ IgemmMaps maps, const IgemmArgs a) {
                 if (lane == 0) {
                     if (PAIR) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl.acc_empty[b]), 0));
                     else mbar_arrive(smem_u32(&ctl.acc_empty[b]));
-                    unsigned int *ticket = a.tickets + (size_t)tile.split * (PAIR ? 8 : 4) + rows32;
-                    order = atomicAdd(ticket, 1u);
-                    if (order == (unsigned)a.parts - 1u) *ticket = 0u;   // for the next launch
+                    order = take_ticket(tile.split);
                 }
                 order = __shfl_sync(0xffffffffu, order, 0);
                 if (order != (unsigned)a.parts - 1u) continue;           // another part of these rows is still to come

@@ -512,7 +512,6 @@ int status_to_code(aet_network *net, const float *pinned3) {
     memcpy(&st, pinned3 + 2, sizeof(int));
     if (st & AET_STATUS_TIMEOUT) {
         cudaMemsetAsync(net->ctx->status_dev, 0, sizeof(int), net->ctx->stream);
-        cudaMemsetAsync(net->ctx->tickets, 0, 2 * kTickets * sizeof(unsigned int), net->ctx->stream);
         aet_set_error("a bounded device-side wait expired during the training step (status %d): the step is incomplete, "
                       "the weights must be reloaded", st);
         return AET_E_TIMEOUT;

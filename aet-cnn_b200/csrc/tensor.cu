@@ -666,7 +666,6 @@ extern "C" int aet_context_check(aet_context *ctx) {
     AET_CUDA(cudaMemcpy(&st, ctx->status_dev, sizeof(int), cudaMemcpyDeviceToHost));
     if (st != 0) {
         cudaMemset(ctx->status_dev, 0, sizeof(int));
-        if (st & AET_STATUS_TIMEOUT) cudaMemset(ctx->tickets, 0, 2 * kTickets * sizeof(unsigned int));   // a part that gave up never took its ticket
         if (st & AET_STATUS_TIMEOUT) {
             aet_set_error("a bounded device-side wait expired (status %d)", st);
             return AET_E_TIMEOUT;
