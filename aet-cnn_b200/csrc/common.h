@@ -501,7 +501,18 @@ bool host_pinned(const void *p);
 int tensor_upload_nchw(aet_context *ctx, float *dev_nhwc, const float *host, int n, int c, int h, int w, int cp);
 int tensor_upload_staged(aet_context *ctx, float *dev_nhwc, const float *dev_nchw, int n, int c, int h, int w, int cp,
                          cudaStream_t stream = nullptr);   // stream: null = the context's
-int tensor_download_staged(aet_context *ctx, const float *dev_nhwc, float *out_nchw, int n, int c, int h, int w, int cp);
+// The last kernel of a prediction leaves the device's status word beside the results (host: page-locked memory, or null): a
+// transfer of its own would cost as much as the whole pass of a small network.
+struct StatusTap {
+    const int *status;
+    int *host;
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ void status_tap(const StatusTap &t) {   // behind pdl_enter: every kernel in front has ended
+    if (t.host && blockIdx.x + blockIdx.y + blockIdx.z + threadIdx.x == 0) *t.host = __ldcg(t.status);
+}
+#endif
+int tensor_download_staged(aet_context *ctx, const float *dev_nhwc, float *out_nchw, int n, int c, int h, int w, int cp, StatusTap tap);
 int tensor_download_nchw(aet_context *ctx, const float *dev_nhwc, float *host, int n, int c, int h, int w, int cp, const float *add = nullptr);
 int tensor_download_nchw_int(aet_context *ctx, const int *dev_nhwc, int *host, int n, int c, int h, int w, int cp);
 int vector_upload(aet_context *ctx, float *dev, const float *host, size_t count);
@@ -576,7 +587,7 @@ int k_param_hash(aet_context *ctx, const float *p, size_t count, uint64_t *hash_
 int k_augment(aet_context *ctx, const float *src_nchw, int n, int c, int sh, int sw, float *dst_nhwc, int size, int cp,
               const aet_augment *params_dev);
 constexpr int kTopkLanes = 32;   // lists of up to this many entries are held by a warp's lanes
-int k_top_k(aet_context *ctx, const float *scores, int samples, int n, int ld, int k, int *index_dev);
+int k_top_k(aet_context *ctx, const float *scores, int samples, int n, int ld, int k, int *index_dev, StatusTap tap = {});
 
 // parameter pointers
 static inline float *layer_W(aet_layer *l) { return l->arena->W + l->seg_w.offset; }

@@ -1658,8 +1658,9 @@ __global__ void augment_kernel(const float *__restrict__ src, int n, int c, int 
 // order.  4 us for one sample of 1000 classes, k = 5.
 constexpr int TOPK_WARPS = 4;
 __global__ void __launch_bounds__(TOPK_WARPS * 32)
-top_k_warp_kernel(const float *__restrict__ scores, int samples, int n, int ld, int k, int *__restrict__ index) {
+top_k_warp_kernel(const float *__restrict__ scores, int samples, int n, int ld, int k, int *__restrict__ index, StatusTap tap) {
     pdl_enter();
+    status_tap(tap);
     const int s = blockIdx.x * TOPK_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (s >= samples) return;
     const float *a = scores + (size_t)s * ld;
@@ -1742,8 +1743,9 @@ top_k_warp_kernel(const float *__restrict__ scores, int samples, int n, int ld, 
     if (lane < k) index[(size_t)s * k + lane] = id;
 }
 // more slots than lanes: one thread per sample runs the loop as it stands
-__global__ void top_k_kernel(const float *__restrict__ scores, int samples, int n, int ld, int k, int *__restrict__ index) {
+__global__ void top_k_kernel(const float *__restrict__ scores, int samples, int n, int ld, int k, int *__restrict__ index, StatusTap tap) {
     pdl_enter();
+    status_tap(tap);
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= samples) return;
     const float *a = scores + (size_t)s * ld;
@@ -2418,13 +2420,13 @@ int k_augment(aet_context *ctx, const float *src_nchw, int n, int c, int sh, int
     return aet_check_launch("augment");
 }
 
-int k_top_k(aet_context *ctx, const float *scores, int samples, int n, int ld, int k, int *index_dev) {
+int k_top_k(aet_context *ctx, const float *scores, int samples, int n, int ld, int k, int *index_dev, StatusTap tap) {
     LaunchScope s(ctx, "top_k", 4.0 * samples * n, 0);
     if (k <= kTopkLanes)
         launch_k(ctx->stream, (unsigned)((samples + TOPK_WARPS - 1) / TOPK_WARPS), TOPK_WARPS * 32, 0, top_k_warp_kernel, scores, samples, n, ld,
-                 k, index_dev);
+                 k, index_dev, tap);
     else
-        launch_k(ctx->stream, (unsigned)((samples + 63) / 64), 64, 0, top_k_kernel, scores, samples, n, ld, k, index_dev);
+        launch_k(ctx->stream, (unsigned)((samples + 63) / 64), 64, 0, top_k_kernel, scores, samples, n, ld, k, index_dev, tap);
     return aet_check_launch("top_k");
 }
 

@@ -504,19 +504,21 @@ int queue_loss_readback(aet_network *net, float *pinned3, cudaStream_t stream = 
     return k_report_loss(net->ctx, sm ? sm->cost_dev : nullptr, pinned3, stream ? stream : net->ctx->stream);
 }
 
-// Turns the status word that came back with a loss into the call's return code.  A timed-out wait leaves the
-// step incomplete (tiles unwritten, the update partly applied): the caller must treat the weights as lost and
+// Turns the status word that came back with a result into the call's return code.  A wait that timed out in a training
+// step leaves it incomplete (tiles unwritten, the update partly applied): the caller must treat the weights as lost and
 // reload a checkpoint.  The non-finite flag is informational and is left for aet_context_check.
-int status_to_code(aet_network *net, const float *pinned3) {
-    int st;
-    memcpy(&st, pinned3 + 2, sizeof(int));
+int status_to_code(aet_network *net, int st, const char *consequence) {
     if (st & AET_STATUS_TIMEOUT) {
         cudaMemsetAsync(net->ctx->status_dev, 0, sizeof(int), net->ctx->stream);
-        aet_set_error("a bounded device-side wait expired during the training step (status %d): the step is incomplete, "
-                      "the weights must be reloaded", st);
+        aet_set_error("a bounded device-side wait expired during %s (status %d)", consequence, st);
         return AET_E_TIMEOUT;
     }
     return AET_OK;
+}
+int step_status(aet_network *net, const float *pinned3) {
+    int st;
+    memcpy(&st, pinned3 + 2, sizeof(int));
+    return status_to_code(net, st, "the training step: the step is incomplete, the weights must be reloaded");
 }
 
 }  // namespace
@@ -948,7 +950,7 @@ extern "C" int aet_network_last_loss(aet_network *net, float *loss) {
         sm->cost_valid = true;
     }
     *loss = net->loss_pinned[1];
-    return status_to_code(net, net->loss_pinned);
+    return step_status(net, net->loss_pinned);
 }
 
 extern "C" int aet_network_train_step(aet_network *net, const float *host_x, const float *host_truth, float *loss) {
@@ -1060,7 +1062,7 @@ extern "C" int aet_network_train_step_async(aet_network *net, const float *host_
     AET_CUDA(cudaEventSynchronize(net->ev_loss[prev]));
     const float *pr = net->loss_pinned + 8 + 4 * prev;
     if (previous_loss) *previous_loss = pr[1];
-    return status_to_code(net, pr);
+    return step_status(net, pr);
 }
 
 // ---------------------------------------------------------------------------- prediction
@@ -1074,6 +1076,18 @@ constexpr size_t kSlotOut = kRingHalf;   // the slot's block: small images in th
 size_t predict_out_bytes(const aet_network *net, int mode, int k) {
     const aet_layer *last = net->layers.back();
     return mode == 0 ? (size_t)net->batch * last->oc * last->oh * last->ow * sizeof(float) : (size_t)net->batch * k * sizeof(int);
+}
+
+// A prediction's status word: in front of the results (the images have left that place when the last kernel writes it).
+int *slot_status(const PredictSlot &s) { return reinterpret_cast<int *>(s.pin + kSlotOut) - 1; }
+int prediction_status(aet_network *net, int st) {
+    return status_to_code(net, st, "this prediction or work queued in front of it: the results are incomplete");
+}
+// the same behind results that did not come by way of a slot
+int prediction_status(aet_network *net) {
+    int st = 0;
+    AET_TRY(vector_download(net->ctx, reinterpret_cast<const float *>(net->ctx->status_dev), reinterpret_cast<float *>(&st), 1));
+    return prediction_status(net, st);
 }
 
 int slot_prepare(aet_network *net, PredictSlot &s) {
@@ -1150,10 +1164,11 @@ int slot_run(aet_network *net, PredictSlot &s, int mode, int k) {
         AET_TRY(net_forward(net, st));
         const aet_layer *last = net->layers.back();
         void *out = s.pin + kSlotOut;
-        if (mode == 0) return tensor_download_staged(ctx, last->output->d, static_cast<float *>(out), last->batch, last->oc, last->oh, last->ow, last->ocp);
-        if (k <= kTopkLanes) return k_top_k(ctx, last->output->d, net->batch, last->oc, last->ocp, k, static_cast<int *>(out));
+        const StatusTap tap = {ctx->status_dev, slot_status(s)};
+        if (mode == 0) return tensor_download_staged(ctx, last->output->d, static_cast<float *>(out), last->batch, last->oc, last->oh, last->ow, last->ocp, tap);
+        if (k <= kTopkLanes) return k_top_k(ctx, last->output->d, net->batch, last->oc, last->ocp, k, static_cast<int *>(out), tap);
         AET_TRY(ctx_scratch(ctx, predict_out_bytes(net, 1, k), &list));   // the forward pass may have moved it
-        AET_TRY(k_top_k(ctx, last->output->d, net->batch, last->oc, last->ocp, k, reinterpret_cast<int *>(list)));
+        AET_TRY(k_top_k(ctx, last->output->d, net->batch, last->oc, last->ocp, k, reinterpret_cast<int *>(list), tap));
         AET_CUDA(cudaMemcpyAsync(out, list, predict_out_bytes(net, 1, k), cudaMemcpyDeviceToHost, ctx->stream));
         return AET_OK;
     });
@@ -1170,7 +1185,8 @@ extern "C" int aet_network_predict(aet_network *net, const float *host_x, float 
         aet_state st = {};
         st.input = net->input; st.train = 0;
         AET_TRY(net_forward(net, st));
-        return aet_tensor_read(net->layers.back()->output, host_out);
+        AET_TRY(aet_tensor_read(net->layers.back()->output, host_out));
+        return prediction_status(net);
     }
     PredictSlot &s = net->predict[0];
     AET_TRY(slot_prepare(net, s));
@@ -1178,7 +1194,7 @@ extern "C" int aet_network_predict(aet_network *net, const float *host_x, float 
     AET_TRY(slot_run(net, s, 0, 0));
     AET_CUDA(cudaStreamSynchronize(net->ctx->stream));
     net->ctx->copier.copy(host_out, s.pin + kSlotOut, out_bytes);
-    return AET_OK;
+    return prediction_status(net, *slot_status(s));
 }
 
 // NNetwork.fuseConvBatchnorm (dnn/NNetwork.c:272-290), the convolutional branch.
@@ -1210,8 +1226,7 @@ int topk_long(aet_network *net, const float *host_x, int k, int *host_indexes) {
     AET_TRY(ctx_scratch(net->ctx, predict_out_bytes(net, 1, k), &scratch));
     AET_TRY(k_top_k(net->ctx, last->output->d, net->batch, last->oc, last->ocp, k, reinterpret_cast<int *>(scratch)));
     AET_CUDA(cudaMemcpyAsync(host_indexes, scratch, predict_out_bytes(net, 1, k), cudaMemcpyDeviceToHost, net->ctx->stream));
-    AET_CUDA(cudaStreamSynchronize(net->ctx->stream));
-    return AET_OK;
+    return prediction_status(net);
 }
 // how many of n samples have their class first, and anywhere, in their list of k
 void count_hits(const int *lists, const int *ids, int n, int k, double *first, double *any) {
@@ -1236,7 +1251,7 @@ extern "C" int aet_network_predict_topk(aet_network *net, const float *host_x, i
     AET_TRY(slot_run(net, s, 1, k));
     AET_CUDA(cudaStreamSynchronize(net->ctx->stream));
     memcpy(host_indexes, s.pin + kSlotOut, predict_out_bytes(net, 1, k));
-    return AET_OK;
+    return prediction_status(net, *slot_status(s));
 }
 
 // The accuracy loop of Classifier.validateSingle (dnn/Classifier.c:359-464) over images already decoded, resized
@@ -1272,11 +1287,12 @@ extern "C" int aet_network_validate(aet_network *net, const float *host_images, 
     for (PredictSlot &s : net->predict) AET_TRY(slot_prepare(net, s));
     AET_CUDA(cudaEventRecord(net->predict[0].done, net->ctx->stream));   // what is queued may still read (or clear) the input tensors
     AET_CUDA(cudaStreamWaitEvent(net->upload_stream, net->predict[0].done, 0));
-    for (int b = 0; b < batches + 2; ++b) {
+    auto batch = [&](int b) -> int {
         PredictSlot &s = net->predict[b & 1];
         if (b >= 2) {   // the slot's results
             const int base = (b - 2) * net->batch, n = count - base < net->batch ? count - base : net->batch;
             AET_CUDA(cudaEventSynchronize(s.done));
+            AET_TRY(prediction_status(net, *slot_status(s)));
             count_hits(reinterpret_cast<const int *>(s.pin + kSlotOut), class_ids + base, n, k, &avg_acc, &avg_topk);
         }
         if (b < batches) {
@@ -1284,6 +1300,15 @@ extern "C" int aet_network_validate(aet_network *net, const float *host_images, 
             AET_TRY(slot_upload(net, s, host_images + (size_t)base * per, n, net->upload_stream));
             AET_TRY(slot_run(net, s, 1, k));
             AET_CUDA(cudaEventRecord(s.done, net->ctx->stream));
+        }
+        return AET_OK;
+    };
+    for (int b = 0; b < batches + 2; ++b) {
+        const int r = batch(b);
+        if (r != AET_OK) {   // nothing may be on its way through the slots when the next call takes them
+            cudaStreamSynchronize(net->upload_stream);
+            cudaStreamSynchronize(net->ctx->stream);
+            return r;
         }
     }
     if (top1) *top1 = (float)(avg_acc / count);

@@ -38,8 +38,9 @@ constexpr size_t kLayoutBlockBytes = 44 * 1024;
 
 template <bool TO_NHWC>
 __global__ void __launch_bounds__(kLayoutThreads)
-layout_pixel_kernel(const float *__restrict__ src, const float *__restrict__ add, float *__restrict__ dst, int n, int c, int hw, int cp) {
+layout_pixel_kernel(const float *__restrict__ src, const float *__restrict__ add, float *__restrict__ dst, int n, int c, int hw, int cp, StatusTap tap) {
     pdl_enter();
+    if (!TO_NHWC) status_tap(tap);
     const size_t e = (size_t)blockIdx.x * kLayoutThreads + threadIdx.x;
     if (e >= (size_t)n * hw) return;
     const size_t b = e / hw, p = e - b * hw;
@@ -72,8 +73,9 @@ layout_pixel_kernel(const float *__restrict__ src, const float *__restrict__ add
 // one image (c * hw floats) per block; the row pitch is odd so that walking along channels hits every bank
 template <bool TO_NHWC>
 __global__ void __launch_bounds__(kLayoutThreads)
-layout_block_kernel(const float *__restrict__ src, const float *__restrict__ add, float *__restrict__ dst, int c, int hw, int cp) {
+layout_block_kernel(const float *__restrict__ src, const float *__restrict__ add, float *__restrict__ dst, int c, int hw, int cp, StatusTap tap) {
     pdl_enter();
+    if (!TO_NHWC) status_tap(tap);
     extern __shared__ float tile[];
     const int pitch = hw | 1;
     const size_t dense = (size_t)blockIdx.x * c * hw, padded = (size_t)blockIdx.x * cp * hw;
@@ -105,8 +107,9 @@ layout_block_kernel(const float *__restrict__ src, const float *__restrict__ add
 // grid: pixel tiles, channel tiles, images (striding over the images past the grid's z limit)
 template <bool TO_NHWC>
 __global__ void __launch_bounds__(kLayoutThreads)
-layout_tile_kernel(const float *__restrict__ src, const float *__restrict__ add, float *__restrict__ dst, int n, int c, int hw, int cp) {
+layout_tile_kernel(const float *__restrict__ src, const float *__restrict__ add, float *__restrict__ dst, int n, int c, int hw, int cp, StatusTap tap) {
     pdl_enter();
+    if (!TO_NHWC) status_tap(tap);
     __shared__ float tile[32][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int p0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
@@ -184,17 +187,17 @@ pull_nchw_kernel(const float4 *__restrict__ src, float *__restrict__ dst, unsign
 }
 
 template <bool TO_NHWC>
-int layout_launch(cudaStream_t stream, const float *src, const float *add, float *dst, int n, int c, int hw, int cp) {
+int layout_launch(cudaStream_t stream, const float *src, const float *add, float *dst, int n, int c, int hw, int cp, StatusTap tap = {}) {
     const size_t block_bytes = (size_t)c * (hw | 1) * sizeof(float);
     if (cp <= 8) {
         const size_t px = (size_t)n * hw;
         launch_k(stream, (unsigned)((px + kLayoutThreads - 1) / kLayoutThreads), kLayoutThreads, 0, layout_pixel_kernel<TO_NHWC>, src, add, dst, n,
-                 c, hw, cp);
+                 c, hw, cp, tap);
     } else if (block_bytes <= kLayoutBlockBytes) {
-        launch_k(stream, (unsigned)n, kLayoutThreads, block_bytes, layout_block_kernel<TO_NHWC>, src, add, dst, c, hw, cp);
+        launch_k(stream, (unsigned)n, kLayoutThreads, block_bytes, layout_block_kernel<TO_NHWC>, src, add, dst, c, hw, cp, tap);
     } else {
         const dim3 grid((hw + 31) / 32, (cp + 31) / 32, n < 65535 ? n : 65535);
-        launch_k(stream, grid, kLayoutThreads, 0, layout_tile_kernel<TO_NHWC>, src, add, dst, n, c, hw, cp);
+        launch_k(stream, grid, kLayoutThreads, 0, layout_tile_kernel<TO_NHWC>, src, add, dst, n, c, hw, cp, tap);
     }
     return aet_check_launch(TO_NHWC ? "nchw_to_nhwc" : "nhwc_to_nchw");
 }
@@ -789,9 +792,9 @@ int tensor_upload_staged(aet_context *ctx, float *dev_nhwc, const float *dev_nch
 }
 
 // Layout change into page-locked host (or device) memory, queued on the context's stream.
-int tensor_download_staged(aet_context *ctx, const float *dev_nhwc, float *out_nchw, int n, int c, int h, int w, int cp) {
+int tensor_download_staged(aet_context *ctx, const float *dev_nhwc, float *out_nchw, int n, int c, int h, int w, int cp, StatusTap tap) {
     ctx->launches++;
-    return layout_launch<false>(ctx->stream, dev_nhwc, nullptr, out_nchw, n, c, h * w, cp);
+    return layout_launch<false>(ctx->stream, dev_nhwc, nullptr, out_nchw, n, c, h * w, cp, tap);
 }
 
 // `add` (may be null): a second tensor of the same layout, added on the way

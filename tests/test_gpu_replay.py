@@ -225,3 +225,27 @@ def test_blocking_stream_is_not_captured_unasked(aet):
         torch.cuda.synchronize()
         torch.cuda.cudart().cudaStreamDestroy(handle.value)
     assert not failed, failed
+
+
+def test_prediction_reports_an_expired_wait(aet):
+    """A bounded wait that ran out is reported by the prediction that follows or contains it, once."""
+    ctx = aet.Context(0)
+    net = cifar(aet, ctx)
+    (x, _), = batches(net, 1)
+    want, best = net.predict(x).copy(), net.predict_topk(x, 3).copy()
+    ids = np.arange(net.batch, dtype=np.int32) % 10
+    share = net.validate(x, ids, 3)
+    try:
+        for call in (lambda: net.predict(x), lambda: net.predict_topk(x, 3), lambda: net.validate(x, ids, 3)):
+            ctx.set_wait_limit(1000000)
+            ctx.wait_probe()
+            with pytest.raises(aet.AetError, match="wait"):
+                call()
+            ctx.set_wait_limit(1000000000)
+            assert np.array_equal(net.predict(x), want) and np.array_equal(net.predict_topk(x, 3), best)
+            assert net.validate(x, ids, 3) == share
+    finally:
+        ctx.set_wait_limit(1000000000)
+    ctx.check()
+    net.close()
+    ctx.close()
