@@ -63,9 +63,21 @@ class Augment(C.Structure):
                 ("flip", C.c_int), ("dhue", C.c_float), ("dsat", C.c_float), ("dexp", C.c_float)]
 
 
-_AUGMENT = np.dtype([(name, np.int32 if kind is C.c_int else np.float32) for name, kind in Augment._fields_])
 _AUGMENT_FORM = "".join("i" if kind is C.c_int else "f" for _, kind in Augment._fields_)
-_augment_fields = operator.itemgetter(*_AUGMENT.names)
+_augment_fields = operator.itemgetter(*(name for name, _ in Augment._fields_))
+
+
+def _pack_augment(params):
+    """The aet_augment records of a list of dicts.  Where every field is there they are packed in one pass (the records have
+    no padding); what that does not take goes field by field: those left out are zero, and a field refuses what its type does."""
+    try:
+        return struct.pack("=" + _AUGMENT_FORM * len(params), *itertools.chain.from_iterable(map(_augment_fields, params)))
+    except (KeyError, TypeError, struct.error, OverflowError):
+        records = (Augment * len(params))()
+        for record, p in zip(records, params):
+            for k, v in p.items():
+                setattr(record, k, v)
+        return bytes(records)
 
 
 class KernelTime(C.Structure):
@@ -472,15 +484,7 @@ class NNetwork:
         """Device-side rotate/crop + flip + HSV distortion of `src` [batch][c][sh][sw] into the network's input tensor;
         `params` is a list of dicts with the aet_augment fields (one per image)."""
         src = _f32(src)
-        try:                      # one pass over the fields; the records are packed without padding
-            form = "=" + _AUGMENT_FORM * len(params)
-            arr = np.frombuffer(struct.pack(form, *itertools.chain.from_iterable(map(_augment_fields, params))), _AUGMENT)
-        except (KeyError, TypeError, struct.error, OverflowError):   # fields left out are zero; other number types
-            arr = np.zeros(len(params), _AUGMENT)
-            for i, p in enumerate(params):
-                for k, v in p.items():
-                    arr[k][i] = v
-        _check(self.L.aet_network_augment_input(self.h, src.ctypes.data, src.shape[2], src.shape[3], arr.ctypes.data))
+        _check(self.L.aet_network_augment_input(self.h, src.ctypes.data, src.shape[2], src.shape[3], _pack_augment(params)))
 
     def fuse_conv_batchnorm(self):
         """NNetwork.fuseConvBatchnorm: fold BN into the convolutions (inference only afterwards)."""

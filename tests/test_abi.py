@@ -85,3 +85,22 @@ def test_every_kernel_waits_for_its_predecessor_before_touching_global_memory():
             assert "pdl_enter()" in src[start:k], "%s: kernel at offset %d never calls pdl_enter()" % (fn, m.start())
             checked += 1
     assert checked >= 30
+
+
+def test_augmentation_draws_are_packed_as_their_types_say(aet):
+    def by_field(params):
+        records = (aet.Augment * len(params))()
+        for r, p in zip(records, params):
+            for k, v in p.items():
+                setattr(r, k, v)
+        return bytes(records)
+
+    full = dict(rad=0.1, scale=1.5, dx=-2, dy=3.25, aspect=1.1, flip=1, dhue=0.05, dsat=1.2, dexp=0.9)
+    for params in ([full, dict(full, flip=0, rad=-0.3)], [full, dict(rad=0.5, flip=True)], [dict(full, label="cat")], [dict(scale=2.0, label=3)],
+                   [dict(full, flip=2 ** 31 + 5)], [dict(full, dx=1e60)], [{}], []):
+        assert aet._pack_augment(params) == by_field(params), params
+    for wrong in (dict(full, flip=0.7), dict(full, rad="0.1"), dict(flip=1.0), dict(full, dexp=None)):
+        with pytest.raises(TypeError):
+            by_field([wrong])
+        with pytest.raises(TypeError):
+            aet._pack_augment([wrong])
