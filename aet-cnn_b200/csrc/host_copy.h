@@ -54,7 +54,7 @@ public:
     // Copies `bytes` from src through the ring of `ring_bytes` (a multiple of kChunk) at `ring`: send(ring offset, source
     // offset, length) is called on the calling thread for consecutive pieces as they are complete (a piece never wraps),
     // and freed() says how many bytes from the start have been consumed, i.e. may be overwritten in the ring.
-    // send returns 0 or an error code, which ends the copy.
+    // send returns 0, freed what it says, or a (negative) error code, which ends the copy.
     template <typename Send, typename Freed>
     int stream(void *ring, size_t ring_bytes, const void *src, size_t bytes, Send send, Freed freed) {
         const size_t ring_chunks = ring_bytes / kChunk, chunks = (bytes + kChunk - 1) / kChunk;
@@ -66,8 +66,12 @@ public:
         int rc = 0;
         while (sent < chunks && rc == 0) {
             if (chunks > ring_chunks && released < sent) {
-                const size_t f = freed();
-                released = f >= bytes ? chunks : f / kChunk;
+                const long long f = freed();
+                if (f < 0) {   // nothing will be consumed any more
+                    rc = (int)f;
+                    break;
+                }
+                released = (size_t)f >= bytes ? chunks : (size_t)f / kChunk;
                 released_.store(released, std::memory_order_release);
             }
             size_t i = next_.load(std::memory_order_relaxed);

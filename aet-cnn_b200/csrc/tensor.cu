@@ -464,20 +464,24 @@ int stage_pieces(aet_context *ctx, void *pin, size_t pin_bytes, const void *host
         if (!ctx->copy_ev[k]) AET_CUDA(cudaEventCreateWithFlags(&ctx->copy_ev[k], cudaEventDisableTiming));
     size_t upto[kCopyEvents] = {0}, freed = 0;
     int head = 0, count = 0;   // events of the pieces in flight, oldest first
-    auto poll = [&]() -> size_t {
-        while (count > 0 && cudaEventQuery(ctx->copy_ev[head]) == cudaSuccess) {
+    auto poll = [&]() -> long long {
+        while (count > 0) {
+            const cudaError_t e = cudaEventQuery(ctx->copy_ev[head]);
+            if (e == cudaErrorNotReady) break;
+            AET_CUDA(e);   // the device has failed: the piece will never be consumed
             freed = upto[head];
             head = (head + 1) % kCopyEvents;
             --count;
         }
-        return freed;
+        return (long long)freed;
     };
     return ctx->copier.stream(pin, pin_bytes, host, bytes, [&](size_t at, size_t lo, size_t len) -> int {
         AET_TRY(launch(static_cast<const char *>(pin) + at, lo, len));
         if (bytes <= pin_bytes) return AET_OK;
         if (count == kCopyEvents) {
             AET_CUDA(cudaEventSynchronize(ctx->copy_ev[head]));
-            poll();
+            const long long f = poll();
+            if (f < 0) return (int)f;
         }
         const int tail = (head + count) % kCopyEvents;
         AET_CUDA(cudaEventRecord(ctx->copy_ev[tail], stream));
