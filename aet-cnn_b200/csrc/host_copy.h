@@ -39,7 +39,7 @@ public:
 
     // Copies `bytes` from src to dst.  `whole`: the size of the copy that this one is a piece of.
     void copy(void *dst, const void *src, size_t bytes, size_t whole = 0) {
-        if (bytes < kParallelFrom) {
+        if (bytes < kParallelFrom || !reserve((bytes + kChunk - 1) / kChunk)) {
             memcpy(dst, src, bytes);
             return;
         }
@@ -54,10 +54,11 @@ public:
     // Copies `bytes` from src through the ring of `ring_bytes` (a multiple of kChunk) at `ring`: send(ring offset, source
     // offset, length) is called on the calling thread for consecutive pieces as they are complete (a piece never wraps),
     // and freed() says how many bytes from the start have been consumed, i.e. may be overwritten in the ring.
-    // send returns 0, freed what it says, or a (negative) error code, which ends the copy.
+    // send returns 0, freed what it says, or a (negative) error code, which ends the copy; `no_memory` is the code for that.
     template <typename Send, typename Freed>
-    int stream(void *ring, size_t ring_bytes, const void *src, size_t bytes, Send send, Freed freed) {
+    int stream(void *ring, size_t ring_bytes, const void *src, size_t bytes, Send send, Freed freed, int no_memory) {
         const size_t ring_chunks = ring_bytes / kChunk, chunks = (bytes + kChunk - 1) / kChunk;
+        if (!reserve(chunks)) return no_memory;
         size_t piece = chunks / 4;   // what is left to send when the copy is done costs time: small pieces, of small copies too
         if (piece > ring_chunks / 4) piece = ring_chunks / 4;
         if (piece < 1) piece = 1;
@@ -91,9 +92,17 @@ public:
     }
 
 private:
+    // Marks for that many chunks; the callers are C entry points, which nothing may leave as an exception.
+    bool reserve(size_t chunks) {
+        try {
+            if (finished_.size() < chunks) finished_ = std::vector<std::atomic<unsigned char>>(chunks);
+        } catch (...) {
+            return false;
+        }
+        return true;
+    }
     void open_job(void *dst, const void *src, size_t bytes, size_t ring_chunks, size_t whole) {
         const size_t chunks = (bytes + kChunk - 1) / kChunk;
-        if (finished_.size() < chunks) finished_ = std::vector<std::atomic<unsigned char>>(chunks);
         for (size_t i = 0; i < chunks; ++i) finished_[i].store(0, std::memory_order_relaxed);
         dst_ = static_cast<unsigned char *>(dst); src_ = static_cast<const unsigned char *>(src);
         bytes_ = bytes; ring_chunks_ = ring_chunks; chunks_ = chunks;

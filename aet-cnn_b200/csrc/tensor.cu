@@ -368,25 +368,22 @@ int ctx_staging(aet_context *ctx, size_t bytes) {
 // page-locked blocks of one size: at most kPoolIdle are kept for the next context, and all are given back when the last
 // context goes.
 namespace {
+constexpr size_t kPoolIdle = 8;
 struct PinnedPool {
     std::mutex m;
-    std::vector<void *> idle;
+    void *idle[kPoolIdle];
+    size_t count = 0;
     int contexts = 0;
 };
-constexpr size_t kPoolIdle = 8;
 PinnedPool &pinned_pool() {
-    static PinnedPool *p = new PinnedPool();   // never destroyed: contexts may outlive static destructors
-    return *p;
+    static PinnedPool p;   // nothing to destroy: contexts may outlive static destructors
+    return p;
 }
 void *pool_take() {
     PinnedPool &p = pinned_pool();
     {
         std::lock_guard<std::mutex> g(p.m);
-        if (!p.idle.empty()) {
-            void *b = p.idle.back();
-            p.idle.pop_back();
-            return b;
-        }
+        if (p.count) return p.idle[--p.count];
     }
     void *b = nullptr;
     if (cudaHostAlloc(&b, 2 * kRingHalf, cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return nullptr; }
@@ -396,8 +393,8 @@ void pool_give(void *b) {
     PinnedPool &p = pinned_pool();
     {
         std::lock_guard<std::mutex> g(p.m);
-        if (p.idle.size() < kPoolIdle) {
-            p.idle.push_back(b);
+        if (p.count < kPoolIdle) {
+            p.idle[p.count++] = b;
             return;
         }
     }
@@ -405,13 +402,15 @@ void pool_give(void *b) {
 }
 void pool_context(int delta) {
     PinnedPool &p = pinned_pool();
-    std::vector<void *> drop;
+    void *drop[kPoolIdle];
+    size_t n = 0;
     {
         std::lock_guard<std::mutex> g(p.m);
         p.contexts += delta;
-        if (p.contexts == 0) drop.swap(p.idle);
+        if (p.contexts == 0)
+            while (p.count) drop[n++] = p.idle[--p.count];
     }
-    for (void *b : drop) cudaFreeHost(b);
+    while (n) cudaFreeHost(drop[--n]);
 }
 }  // namespace
 void *pinned_block_take() { return pool_take(); }
@@ -488,7 +487,7 @@ int stage_pieces(aet_context *ctx, void *pin, size_t pin_bytes, const void *host
         upto[tail] = lo + len;
         ++count;
         return AET_OK;
-    }, poll);
+    }, poll, AET_E_NOMEM);
 }
 unsigned pull_blocks(size_t floats) { return (unsigned)((floats + kLayoutThreads * 8 - 1) / (kLayoutThreads * 8)); }
 // the context's ring as a whole, for one upload that is the next thing on the stream

@@ -6,7 +6,17 @@ from conftest import ROOT
 
 PROGRAM = r"""
 #include "host_copy.h"
+#include <new>
 #include <stdio.h>
+#include <stdlib.h>
+
+static bool full = false;   // memory has run out
+void *operator new(size_t n) {
+    if (full) throw std::bad_alloc();
+    return malloc(n);
+}
+void operator delete(void *p) noexcept { free(p); }
+void operator delete(void *p, size_t) noexcept { free(p); }
 
 #define CHECK(x) do { if (!(x)) { printf("line %d: %s\n", __LINE__, #x); return 1; } } while (0)
 
@@ -37,18 +47,26 @@ int main() {
                     const size_t f = freed;
                     freed = before == f ? sent : before;
                     return (long long)f;
-                });
+                }, -7);
             CHECK(rc == 0 && sent == n && memcmp(dst.data(), src.data(), n) == 0);
         }
     // a consumer that fails: the copy ends with its code, whoever finds out
     int calls = 0;
     CHECK(copier.stream(ring.data(), ring_bytes, src.data(), src.size(), [&](size_t, size_t, size_t) { return 0; },
-                        [&]() -> long long { return ++calls > 5 ? -2 : 0; }) == -2);
+                        [&]() -> long long { return ++calls > 5 ? -2 : 0; }, -7) == -2);
     size_t gone = 0;
     CHECK(copier.stream(ring.data(), ring_bytes, src.data(), src.size(), [&](size_t, size_t lo, size_t len) { gone = lo + len; return lo > 0 ? -3 : 0; },
-                        [&]() -> long long { return (long long)gone; }) == -3);
+                        [&]() -> long long { return (long long)gone; }, -7) == -3);
     copier.copy(dst.data(), src.data(), src.size());
     CHECK(memcmp(dst.data(), src.data(), src.size()) == 0);
+    // without memory for its marks a copy is made alone, and a stream is refused before anything was sent
+    HostCopier fresh;
+    std::fill(dst.begin(), dst.end(), 0);
+    full = true;
+    fresh.copy(dst.data(), src.data(), src.size());
+    const int rc = fresh.stream(ring.data(), ring_bytes, src.data(), src.size(), [&](size_t, size_t, size_t) { return -9; }, [&]() -> long long { return 0; }, -7);
+    full = false;
+    CHECK(rc == -7 && memcmp(dst.data(), src.data(), src.size()) == 0);
     return 0;
 }
 """
