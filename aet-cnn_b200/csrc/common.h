@@ -554,6 +554,7 @@ int k_stem_gram(aet_layer *l, const float *x_in);
 int k_stem_backward(aet_layer *l, aet_layer *pool, const float *x_in);
 int k_stem_finish(aet_layer *l, float *dw, int accumulate);
 int k_stem_delta(aet_layer *l, aet_layer *pool);
+int k_zero_pads(aet_layer *l);
 int k_bias_act_backward(aet_layer *l, aet_layer *pool = nullptr);
 bool pool_bias_backward_ok(const aet_layer *pool);
 int k_maxpool_forward(aet_layer *l, const float *x);

@@ -2445,6 +2445,24 @@ int k_report_loss(aet_context *ctx, const float *cost2, float *pinned3, cudaStre
     return aet_check_launch("report_loss");
 }
 
+namespace {
+__global__ void __launch_bounds__(TB) zero_pads_kernel(float *y, long long pixels, int c, int cp) {
+    pdl_enter();
+    const long long p = (long long)blockIdx.x * TB + threadIdx.x;
+    if (p >= pixels) return;
+    for (int k = c; k < cp; ++k) y[(size_t)p * cp + k] = 0.f;
+}
+}  // namespace
+// The channels that pad a convolution's output hold act(0).  Where that is not zero they are cleared: the next layer's weight
+// gradient would see them, its update would give their weights values, and its next forward pass would count them in.
+int k_zero_pads(aet_layer *l) {
+    if (l->ocp == l->oc || act_forward(0.f, l->act) == 0.f) return AET_OK;
+    const long long pixels = (long long)l->batch * l->oh * l->ow;
+    LaunchScope s(l->ctx, "zero_pads", 4.0 * pixels * (l->ocp - l->oc), 0);
+    launch_k(l->ctx->stream, (unsigned)((pixels + TB - 1) / TB), TB, 0, zero_pads_kernel, l->output->d, pixels, l->oc, l->ocp);
+    return aet_check_launch("zero_pads");
+}
+
 int k_param_hash(aet_context *ctx, const float *p, size_t count, uint64_t *hash_dev) {
     LaunchScope s(ctx, "param_hash", 4.0 * count, 0);
     launch_k(ctx->stream, (unsigned)((count + TB - 1) / TB), TB, 0, param_hash_kernel, p, count,

@@ -322,6 +322,7 @@ extern "C" void aet_layer_destroy(aet_layer *l) {
 int layer_form_output(aet_layer *l) {
     if (l->output_stale) {   // fused forward skipped the full-resolution output
         AET_TRY(k_bn_apply(l, l->last_forward_train ? 0 : 1));
+        AET_TRY(k_zero_pads(l));
         l->output_stale = false;
     }
     if (l->lin_out_stale) {  // the linear head never ran the convolution itself
@@ -396,6 +397,7 @@ extern "C" int aet_layer_forward(aet_layer *l, aet_state state) {
                 pool->output->lazy_zero = false;
             } else {
                 AET_TRY(k_bn_apply(l, state.train ? 0 : 1));
+                AET_TRY(k_zero_pads(l));
                 l->output_stale = false;
             }
         } else {
@@ -410,6 +412,7 @@ extern "C" int aet_layer_forward(aet_layer *l, aet_state state) {
             }
             l->lin_fwd_pending = false;
             AET_TRY(conv_fprop(l, state.input->d, l->output->d, layer_b(l), 1));
+            AET_TRY(k_zero_pads(l));
         }
         l->output->lazy_zero = false;
         return AET_OK;

@@ -900,3 +900,56 @@ def test_weights_file_partial_loads(aet, ctx, oracle):
         assert np.array_equal(net.layer(1).read(aet.P_WEIGHTS), init[1]) and np.array_equal(net.layer(2).read(aet.P_WEIGHTS), init[2])
         net.close()
     src.close()
+
+
+LIFTED_CFG = """[net]
+batch=4
+width=12
+height=12
+channels=3
+learning_rate=0.1
+momentum=0.9
+decay=0.0005
+policy=constant
+[convolutional]
+filters=6
+size=3
+pad=1
+batch_normalize=%d
+activation=%s
+[convolutional]
+filters=5
+size=3
+pad=1
+batch_normalize=%d
+activation=%s
+[convolutional]
+filters=10
+size=1
+activation=linear
+[avgpool]
+[softmax]
+"""
+
+
+@pytest.mark.parametrize("act", ["logistic", "plse"])
+@pytest.mark.parametrize("bn", [0, 1])
+def test_activations_that_lift_zero_leave_the_pad_channels_empty(aet, ctx, oracle64, tmp_path, act, bn):
+    """Filter counts that are no multiple of four, activations that are not zero at zero: what the channels that only pad
+    the tensors held would reach the next layer's weights with its first update.  Smooth (or nearly so) functions in
+    3xTF32: the steps stay within the 1e-5 of a pass, a few times over."""
+    cfg = tmp_path / "lifted.cfg"
+    cfg.write_text(LIFTED_CFG % (bn, act, bn, act))
+    ctx.set_math(aet.MATH_3XTF32)
+    try:
+        net, onet, opts, specs = build_pair(aet, ctx, oracle64, str(cfg), 4)
+        for step in range(6):
+            x, truth = batch_for(opts, 10, 4, 77, step)
+            loss = net.train(x, truth)
+            oloss = onet.train_step(x, truth, opts["learning_rate"], opts["momentum"], opts["decay"])
+            assert abs(loss - oloss) <= 1e-4 * abs(oloss), (step, loss, oloss)
+        for i in range(3):
+            assert rel_l2(net.layer(i).read(aet.P_WEIGHTS), onet.param(i, ob.P_WEIGHTS)) <= 1e-4, i
+        net.close()
+    finally:
+        ctx.set_math(aet.MATH_TF32)
