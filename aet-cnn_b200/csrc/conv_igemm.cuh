@@ -53,7 +53,7 @@ struct IgemmArgs {
     int tap_step;               // taps of a class are this far apart in the filter (data gradient: the stride)
     int dil, S;
     int scatter, H, W;          // data gradient with a stride: rows go to pixels (s * i + ph, s * j + pw)
-    int inner, slabs_per_tap;   // channels of the K dimension
+    int slabs_per_tap;          // 32-channel slabs of the K dimension
     int b_blocks;               // data gradient, channel counts that are no multiple of 32: one copy per 32-channel block (0: one copy)
     int n_tiles, m_tiles;
     // The tiles past the last whole round (or all of them, when there are few) are cut into `parts` along K, so that every
@@ -600,6 +600,11 @@ IgemmPlan igemm_plan(const aet_context *ctx, const int *rows, int classes, int s
     return best;
 }
 
+// "i2c_", p(air) or n(o pair), filters (or channels) of a tile
+void igemm_label(char *variant, size_t size, const IgemmPlan &plan, bool x3) {
+    snprintf(variant, size, "i2c_%s%d%s", plan.pair ? "p" : "n", plan.bn, x3 ? "_x3" : "");
+}
+
 template <int KIND, bool PAIR, bool X3>
 int igemm_launch(aet_context *ctx, const IgemmMaps &maps, IgemmArgs &a, const char *name, const char *variant, double flops) {
     const int bnc = PAIR ? a.bn / 2 : a.bn;
@@ -623,10 +628,11 @@ int igemm_launch(aet_context *ctx, const IgemmMaps &maps, IgemmArgs &a, const ch
 }
 
 template <int KIND>
-int igemm_run(aet_layer *l, const ConvArgs &ca, const IgemmPlan &plan, const IgemmMaps &maps, IgemmArgs &a, const char *name,
-              const char *variant, double flops) {
+int igemm_run(aet_layer *l, const ConvArgs &ca, const IgemmPlan &plan, const IgemmMaps &maps, IgemmArgs &a, const char *name, double flops) {
     aet_context *ctx = l->ctx;
     const bool x3 = ctx->math == AET_MATH_3XTF32;
+    char variant[32];
+    igemm_label(variant, sizeof(variant), plan, x3);
     a.direct_tiles = plan.direct; a.parts = plan.parts;
     if (plan.parts > 1) {
         // the batch statistics' partial rows (already handed out at the arena's start) stay in front of the parts
@@ -683,12 +689,9 @@ int igemm_fprop(aet_layer *l, const ConvArgs &a, double flops) {
     c.tile_end = t.m_tiles = (a.n_rows + (plan.pair ? 255 : 127)) / (plan.pair ? 256 : 128);
     t.classes = 1; t.out = a.out; t.bias = a.bias; t.act = a.act; t.stat_shift = a.stat_shift; t.stat_partial = a.stat_partial;
     t.bn = plan.bn; t.n_cols = a.n_cols; t.out_ld = a.out_ld; t.step = g.sx; t.tap_step = 1; t.dil = g.dil; t.S = g.S;
-    t.inner = g.cp; t.slabs_per_tap = slabs_per_tap; t.n_tiles = (a.n_cols + plan.bn - 1) / plan.bn;
+    t.slabs_per_tap = slabs_per_tap; t.n_tiles = (a.n_cols + plan.bn - 1) / plan.bn;
     if (a.stat_rows_out) *a.stat_rows_out = t.m_tiles * (plan.pair ? 8 : 4);
-    char variant[32];
-    if (g.sx == 1 && g.dil == 1 && l->groups == 1 && !x3) snprintf(variant, sizeof(variant), "ragged");
-    else snprintf(variant, sizeof(variant), "i2c_%s%d%s", plan.pair ? "p" : "n", plan.bn, x3 ? "_x3" : "");
-    return igemm_run<KIND_FPROP>(l, a, plan, maps, t, "conv_fprop_tma", variant, flops);
+    return igemm_run<KIND_FPROP>(l, a, plan, maps, t, "conv_fprop_tma", flops);
 }
 
 int igemm_dgrad(aet_layer *l, const ConvArgs &a, double flops) {
@@ -752,12 +755,9 @@ int igemm_dgrad(aet_layer *l, const ConvArgs &a, double flops) {
     }
     t.out = a.out; t.act = AET_LINEAR; t.bn = plan.bn; t.n_cols = a.n_cols; t.out_ld = a.out_ld;
     t.step = 1; t.tap_step = s; t.dil = s == 1 ? g.dil : 1; t.S = g.S; t.scatter = s; t.H = g.H; t.W = g.W;
-    t.inner = g.kp; t.slabs_per_tap = slabs_per_tap; t.b_blocks = blocks32 ? 0 : bnc / 32;
+    t.slabs_per_tap = slabs_per_tap; t.b_blocks = blocks32 ? 0 : bnc / 32;
     t.n_tiles = (a.n_cols + plan.bn - 1) / plan.bn;
-    char variant[32];
-    if (s == 1 && g.dil == 1 && l->groups == 1 && !x3) snprintf(variant, sizeof(variant), "ragged");
-    else snprintf(variant, sizeof(variant), "i2c_%s%d%s", plan.pair ? "p" : "n", plan.bn, x3 ? "_x3" : "");
-    return igemm_run<KIND_DGRAD>(l, a, plan, maps, t, "conv_dgrad_tma", variant, flops);
+    return igemm_run<KIND_DGRAD>(l, a, plan, maps, t, "conv_dgrad_tma", flops);
 }
 
 }  // namespace

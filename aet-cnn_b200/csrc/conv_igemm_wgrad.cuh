@@ -351,10 +351,7 @@ int igemm_wgrad(aet_layer *l, const ConvArgs &ca, float *dw, int accumulate, dou
     if (!direct) AET_TRY(ctx_scratch(ctx, out_floats * t.splits * sizeof(float), &t.out));
     float *partial = t.out;
     char variant[32];
-    cuuint32_t bw, bh, bi;
-    if (g.sx != 1 || g.dil != 1 || l->groups != 1 || x3) snprintf(variant, sizeof(variant), "i2c_%s%d%s", plan.pair ? "p" : "n", plan.bn, x3 ? "_x3" : "");
-    else if (pixel_box(BK, g.OH, g.OW, &bw, &bh, &bi)) variant[0] = 0;
-    else snprintf(variant, sizeof(variant), g.OW > BK ? "wide" : "ragged");
+    igemm_label(variant, sizeof(variant), plan, x3);
     int r;
     if (x3) r = plan.pair ? igemm_wgrad_launch<true, true>(ctx, mx, *mdy, t, variant, flops) : igemm_wgrad_launch<false, true>(ctx, mx, *mdy, t, variant, flops);
     else if (plan.pair) r = igemm_wgrad_launch<true, false>(ctx, mx, *mdy, t, variant, flops);

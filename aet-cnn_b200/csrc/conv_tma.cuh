@@ -521,7 +521,7 @@ int tma_fprop(aet_layer *l, const ConvArgs &a, double flops, bool cluster_only =
         AET_TRY(launch_tma<KIND_FPROP>(l->ctx, ma, mb, t, grid, "conv_fprop_tma.ks", flops));
         return launch_fprop_reduce(l->ctx, partial, a.out, a.bias, out_floats, a.out_ld, splits, a.act);
     }
-    return launch_tma<KIND_FPROP>(l->ctx, ma, mb, t, grid, per_img ? "conv_fprop_tma.ragged" : (parts ? "conv_fprop_tma.cl" : "conv_fprop_tma"), flops);
+    return launch_tma<KIND_FPROP>(l->ctx, ma, mb, t, grid, parts ? "conv_fprop_tma.cl" : (per_img ? "conv_fprop_tma.ragged" : "conv_fprop_tma"), flops);
 }
 
 int tma_dgrad(aet_layer *l, const ConvArgs &a, double flops, bool cluster_only = false) {
@@ -584,7 +584,7 @@ int tma_dgrad(aet_layer *l, const ConvArgs &a, double flops, bool cluster_only =
         t.cluster = parts;
         t.slabs_per_split = (t.total_slabs + parts - 1) / parts;
         grid.z = parts;
-        return launch_tma<KIND_DGRAD>(l->ctx, ma, mb, t, grid, per_img ? "conv_dgrad_tma.ragged" : "conv_dgrad_tma.cl", flops);
+        return launch_tma<KIND_DGRAD>(l->ctx, ma, mb, t, grid, "conv_dgrad_tma.cl", flops);
     }
     if (a.stat_rows_out) *a.stat_rows_out = (int)grid.x;   // only the forward launcher is given one
     const int splits = per_img ? 1 : fd_splits(l->ctx, (int)(grid.x * grid.y), t.total_slabs);

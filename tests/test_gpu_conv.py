@@ -90,21 +90,26 @@ def test_conv_tma_tf32(aet, ctx, oracle, shape):
 
 
 # Maps whose rows do not divide the 128-pixel tile / 32-pixel slab (the 27x27 and 13x13 maps of an AlexNet-style
-# network): the TMA kernels tile them as whole rows of one image and leave the rest of the tile unused.
+# network).  Tensors of 128 KB and more are walked in im2col mode (i2c), smaller ones are tiled as whole rows of one
+# image with the rest of the tile unused (ragged; rows wider than a slab: wide), and a few images with a long K loop are
+# shared by clusters (cl).  Beside each shape: what runs forward, for the data gradient and for the weight gradient.
 RAGGED_SHAPES = [
-    (4, 96, 27, 27, 256, 5, 1, 2, 1),      # AlexNet-style conv 2: 5x5, 4 rows per tile, 7 tiles per image (the last one 3 rows)
-    (4, 256, 13, 13, 384, 3, 1, 1, 1),     # conv 3: 9 rows per tile, 2 tiles per image; 384 filters = three 128-filter tiles
-    (5, 384, 13, 13, 256, 3, 1, 1, 2),     # conv 5
-    (3, 64, 13, 13, 64, 3, 1, 1, 2),       # one N tile, odd batch
-    (2, 32, 7, 20, 32, 3, 1, 1, 0),        # non-square: 6 + 1 rows
-    (2, 64, 9, 100, 32, 1, 1, 0, 1),       # one row per tile (w > 64), 1x1
-    (2, 32, 12, 40, 64, 3, 1, 1, 2),       # rows wider than a weight-gradient K slab: two 32-column slabs per row
-    (1, 64, 56, 56, 64, 3, 1, 1, 1),       # a 56x56 map (ResNet-style): two rows per forward tile, 32 + 24 columns per slab pair
+    ((4, 96, 27, 27, 256, 5, 1, 2, 1), "i2c i2c i2c"),          # AlexNet-style conv 2: 5x5
+    ((4, 256, 13, 13, 384, 3, 1, 1, 1), "i2c cl i2c"),          # conv 3: 384 filters
+    ((5, 384, 13, 13, 256, 3, 1, 1, 2), "i2c cl i2c"),          # conv 5
+    ((3, 64, 13, 13, 64, 3, 1, 1, 2), "cl cl ragged"),          # one N tile, odd batch
+    ((2, 32, 7, 20, 32, 3, 1, 1, 0), "ragged ragged ragged"),   # non-square: 6 + 1 rows
+    ((2, 64, 9, 100, 32, 1, 1, 0, 1), "ragged i2c i2c"),        # one row per tile (w > 64), 1x1
+    ((2, 32, 12, 40, 64, 3, 1, 1, 2), "ragged cl wide"),        # rows wider than a weight-gradient K slab: two 32-column slabs per row
+    ((1, 64, 56, 56, 64, 3, 1, 1, 1), "cl cl i2c"),             # a 56x56 map (ResNet-style): two rows per forward tile
+    ((3, 32, 13, 13, 32, 3, 1, 1, 1), "ragged ragged ragged"),  # 9 + 4 rows
+    ((1, 32, 27, 27, 64, 1, 1, 0, 1), "ragged i2c ragged"),     # 4 rows per tile, 7 tiles per image (the last one 3 rows)
+    ((2, 32, 7, 50, 32, 3, 1, 1, 1), "ragged ragged wide"),     # two rows per tile; 32 + 18 columns per slab pair
 ]
 
 
-@pytest.mark.parametrize("shape", RAGGED_SHAPES)
-def test_conv_tma_ragged_maps(aet, ctx, oracle, shape):
+@pytest.mark.parametrize("shape,kernels", RAGGED_SHAPES)
+def test_conv_tma_ragged_maps(aet, ctx, oracle, shape, kernels):
     ctx.set_math(aet.MATH_TF32)
     ctx.profile(1)
     try:
@@ -112,11 +117,9 @@ def test_conv_tma_ragged_maps(aet, ctx, oracle, shape):
         used = variants_used(ctx)
     finally:
         ctx.profile(0)
-    names = {u.split("#")[0] for u in used}
-    want = {"conv_fprop_tma.ragged", "conv_dgrad_tma.ragged"}
-    # a weight-gradient K slab is 32 pixels: narrower maps are tiled as whole rows, wider ones as 32-column pieces of a row
-    want.add("conv_wgrad_tma.ragged" if shape[3] <= 32 else "conv_wgrad_tma.wide")
-    assert want <= names, sorted(names)
+    names = {u.split("#")[0].split("_n")[0].split("_p")[0] if ".i2c_" in u else u.split("#")[0] for u in used}
+    want = {"conv_%s_tma.%s" % (kind, variant) for kind, variant in zip(("fprop", "dgrad", "wgrad"), kernels.split())}
+    assert want <= names, sorted(used)
     check(got, ref, TOL_TF32)
     # and the same shapes with the option off go to the gather kernel and agree with it closely
     ctx.set_option("ragged", 0)

@@ -540,9 +540,9 @@ groups=1
 
 
 def test_batchnorm_statistics_from_ragged_tiles(aet, ctx, oracle):
-    """BN convolutions on 13x13 maps: the TMA forward kernel tiles each image as 9 + 4 rows and its epilogue's batch
-    statistics must count exactly the pixels that exist.  Default TF32 math against the oracle: means, variances,
-    outputs, weight gradients."""
+    """BN convolutions on 13x13 maps: the first layer's tiles are 9 + 4 rows of an image, the second one's (a tensor large enough
+    for im2col mode) 128 consecutive pixels with a last tile that is partly empty; the epilogue's batch statistics must
+    count exactly the pixels that exist.  Default TF32 math against the oracle: means, variances, outputs, weight gradients."""
     from oracle import cfgfile
     import aet_cnn_b200.synth as synth
     batch = 6
@@ -562,9 +562,11 @@ def test_batchnorm_statistics_from_ragged_tiles(aet, ctx, oracle):
     ctx.profile(1)
     net.forward(aet.make_state(input=net.input, truth=net.truth, train=1))
     net.backward(aet.make_state(input=net.input, truth=net.truth, train=1))
-    names = {r["name"].split("#")[0] for r in ctx.profile_read()}
+    used = {r["name"] for r in ctx.profile_read()}
     ctx.profile(0)
-    assert {"conv_fprop_tma.ragged", "conv_dgrad_tma.ragged", "conv_wgrad_tma.ragged"} <= names, sorted(names)
+    assert {"conv_fprop_tma.ragged#0", "conv_wgrad_tma.ragged#0", "conv_dgrad_tma.ragged#1"} <= used, sorted(used)
+    assert any(n.startswith("conv_fprop_tma.i2c_") and n.endswith("#1") for n in used), sorted(used)
+    names = {n.split("#")[0] for n in used}
     assert "bn_stats" not in names, sorted(names)      # the statistics came out of the convolution's epilogue
     onet.forward(x, truth); onet.backward(x)
     ctx.check()
