@@ -42,9 +42,12 @@ struct ConvArgs {
     const float *src_b;   // fprop: w      dgrad: w       wgrad: x
     float *out;           // fprop: y      dgrad: dx      wgrad: split-K partials
     const float *bias;    // fprop epilogue, may be null
-    const float *stat_shift;   // fprop: accumulate batch-norm statistics of the output around this per-channel shift
-    float *stat_partial;       //        into one row [2][out_ld] per CTA along M (null: off)
-    int *stat_rows_out;        // host side: the launcher stores the number of partial rows (its grid.x) here
+    // fprop: batch-norm statistics of the output around this per-channel shift, summed into partial rows [2][out_ld] (null:
+    // off).  A launcher writes at most four rows per 128 output pixels and four more (`stats->floats` is the room), stores
+    // how many, and may move them to another place (`stats->partial`).
+    const float *stat_shift;
+    float *stat_partial;
+    int *stat_rows_out;        // host side: the number of partial rows
     ConvStats *stats;          // host side: owner of the partial rows (null: off)
     int act;              // fprop epilogue activation
     int bn;               // N tile (multiple of 16, <= 256)
