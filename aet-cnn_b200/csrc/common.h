@@ -302,7 +302,6 @@ struct PredictSlot {
     float *dev_in = nullptr;
     cudaEvent_t uploaded = nullptr, done = nullptr;
     PassGraph graph[2];
-    int k = 0;
 };
 
 struct aet_network {
@@ -349,6 +348,7 @@ struct aet_network {
     PassGraph graph[4];
     PredictSlot predict[2];
     EagerRuns eager[2], predict_eager[2];
+    int topk = 0;                                              // list length of the top-k passes that were last run
     cudaStream_t upload_stream = nullptr;                      // uploads of a validation loop's next batch
     int cur_slot = 0;                                          // input slot of the step being queued
     aet_tensor *input_alt = nullptr, *truth_alt = nullptr;     // slot 1 (slot 0 = `input`, `truth`)

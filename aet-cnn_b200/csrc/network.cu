@@ -929,7 +929,10 @@ extern "C" int aet_network_train_step_device(aet_network *net, float *loss) {
     const int gi = kind + 2 * net->cur_slot;   // a graph holds its tensors' addresses: one per input slot
     const bool clean_now = net->subdivisions == 1 && net->grad_clean;
     PassGraph &g = net->graph[gi];
-    if (g.exec && net->graph_clean[gi] != clean_now) graph_release(g);   // captured in the other arena state
+    if (g.exec && net->graph_clean[gi] != clean_now) {   // captured in the other arena state
+        graph_release(g);
+        if (net->use_graph != 1) net->eager[kind] = EagerRuns();
+    }
     net->graph_clean[gi] = clean_now;
     const int first_capture = net->use_graph == 1 ? 1 : (net->use_graph == 2 && !net->comm ? 8 : -1);
     AET_TRY(run_pass(net, g, net->eager[kind], first_capture, net->use_graph == 1, true, [&] { return run_step(net, final); }));
@@ -1148,7 +1151,11 @@ int slot_upload(aet_network *net, PredictSlot &s, const float *host, int images,
 // Queues the pass over the slot's images; results land in the slot's block.  mode 0: scores, 1: top-k indexes.
 int slot_run(aet_network *net, PredictSlot &s, int mode, int k) {
     aet_context *ctx = net->ctx;
-    if (mode == 1 && s.k != k) { graph_release(s.graph[1]); s.k = k; }
+    if (mode == 1 && net->topk != k) {   // another pass: captured when it has run like any other
+        for (PredictSlot &q : net->predict) graph_release(q.graph[1]);
+        net->predict_eager[1] = EagerRuns();
+        net->topk = k;
+    }
     net->input->touched = true;
     float *list = nullptr;   // the long lists are worked on in memory, not across the link (sized here: a capture cannot allocate)
     if (mode == 1 && k > kTopkLanes) AET_TRY(ctx_scratch(ctx, predict_out_bytes(net, 1, k), &list));
