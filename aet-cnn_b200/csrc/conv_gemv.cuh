@@ -8,6 +8,10 @@
 
 namespace {
 
+// Medians by events, cold L2 (us), this kernel at 1, 2, 3 and 4 images / the padded tile and its sum at 5, 6 and 8:
+//   9216 -> 4096:  34.5  38.4  40.6  43.7 / 58.6  58.3  58.3      4096 -> 4096:  20.6  21.4  23.2  24.6 / 38.0  35.9  35.6
+//   4096 -> 1000:  11.1  12.6  12.7  13.2 / 23.9  24.7  24.7       512 -> 10:     8.1   7.4   7.3   7.8 / 13.0  13.0  13.0
+// An image costs 3 us of the largest layer, so the kernel would hold a few images longer; it is built for up to four.
 constexpr int GEMV_MAX_IMAGES = 4;
 constexpr int GEMV_THREADS = 256, GEMV_FILTERS = 2;   // filters per block; its eight warps share their channels
 

@@ -18,11 +18,12 @@
 // do, closes the job when none is left, and waits only for helpers that are inside a chunk.
 class HostCopier {
 public:
-    // Waking a sleeping thread costs the waker about 10 us and the woken one 30 to 50 us (virtual machines): a copy has to
-    // take several times that on one core before it is worth sharing.
+    // Waking a sleeping thread costs the waker about 10 us and the woken one 30 to 50 us (virtual machines), so all helpers
+    // are woken only for a copy that takes several times that on one core.
     static constexpr size_t kWakeFrom = 4 * 1024 * 1024;
     // Two helpers stay awake for a millisecond after a job, which is longer than a serving or training loop takes to come
-    // back; while they are, smaller copies are shared too (1.5 MB: 76 us alone).
+    // back; while they are, smaller copies are shared too (1.5 MB: 76 us alone).  With nobody awake a copy from here on
+    // wakes one helper, 10 us that the copy itself gets little for: it is for the copies that follow.
     static constexpr size_t kParallelFrom = 512 * 1024;
     static constexpr int kHelpers = 5, kLingering = 2;   // six copying threads saturate the host's memory on this path
     static constexpr size_t kChunk = 128 * 1024;

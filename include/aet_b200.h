@@ -93,7 +93,11 @@ typedef struct aet_state {
 
 /* ------------------------------------------------------------------ context
  * Replaces the MtcsTool / MtcsStream / MtcsMem singletons (call sites mtcs/MtcsTool.c:22-30,
- * mtcs/MtcsIOData.c:21,47-51).  One context = one device + one stream + one scratch arena. */
+ * mtcs/MtcsIOData.c:21,47-51).  One context = one device + one stream + one scratch arena.
+ * Pageable host data goes through page-locked staging memory, in both directions.  The first such copy of 512 KB or more of a
+ * context starts helper threads (at most five, and one fewer than the processors of the host) that share these copies with
+ * the calling thread and end with the context.  They sleep between copies, except that two of them stay awake, spinning,
+ * for a millisecond after each. */
 const char  *aet_last_error(void);
 const char  *aet_version(void);
 aet_context *aet_context_create(int device);
@@ -233,7 +237,9 @@ int   aet_network_last_loss(aet_network *net, float *loss);
  * aet_network_last_loss drains the pipeline.  The first call allocates the two staging slots.
  * Returns AET_E_TIMEOUT when the previous step's kernels gave up a bounded wait. */
 int   aet_network_train_step_async(aet_network *net, const float *host_x, const float *host_truth, float *previous_loss);
-/* NNetwork.predict (dnn/NNetwork.c:411-428): forward with train=0, copy the last layer's output. */
+/* NNetwork.predict (dnn/NNetwork.c:411-428): forward with train=0, copy the last layer's output.  This call,
+ * aet_network_predict_topk and aet_network_validate return AET_E_TIMEOUT when a bounded device-side wait expired in the pass
+ * or in work queued in front of it. */
 int   aet_network_predict(aet_network *net, const float *host_x, float *host_out);
 /* NNetwork.fuseConvBatchnorm (dnn/NNetwork.c:272-290, dnn/ConvolutionalLayer.c:983-1003): folds every batch-norm
  * layer's rolling statistics and scale into its convolution's biases and weights; afterwards the network only
@@ -260,8 +266,10 @@ typedef struct aet_augment {
     float dhue, dsat, dexp;             /* distort(dhue, dsat, dexp); ignored unless channels == 3 */
 } aet_augment;
 int   aet_network_augment_input(aet_network *net, const float *host_src, int src_h, int src_w, const aet_augment *params);
-/* Capture forward+backward+update into a CUDA graph that later train steps replay (0 = off, for predictions too; without a
- * call a network on one GPU captures its steps after eight equal ones). */
+/* Capture forward+backward+update into a CUDA graph that later train steps replay (0 = off, for predictions too).  Without a
+ * call a network on one GPU captures its steps after eight equal ones, and predictions from the second one of a kind on, where
+ * the context's stream can be captured and does not synchronise with the legacy default stream; what cannot be captured runs
+ * as plain launches.  After a call with 1 a training step that cannot be captured is an error. */
 int   aet_network_use_graph(aet_network *net, int enable);
 /* NNetwork.loadWeights / saveWeights (dnn/NNetwork.c:64-147): Darknet .weights container. */
 int   aet_network_load_weights(aet_network *net, const char *path);
