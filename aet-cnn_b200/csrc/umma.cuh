@@ -49,6 +49,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 // Wall-clock limit of every device-side wait (nanoseconds); one second unless the host changes it
 // (cudaMemcpyToSymbol, per device).  Read only on the slow path of a wait.
 __constant__ unsigned long long g_wait_limit_ns = 1000000000ull;
+// Copies and MMAs that are on their way when a wait runs out still write this CTA's shared memory and TMEM.  Their barriers
+// cannot be asked (a phase that misses another role's arrival never completes), so the thread that gives up stays for two
+// milliseconds, hundreds of times what a copy takes, and its CTA (and cluster) with it: every role joins it before the end.
+constexpr unsigned long long kLandingNs = 2000000ull;
 
 // Waits for the phase with the given parity.  `abort_flag` lives in shared memory: once any
 // role of the CTA has given up, the others leave their waits quickly as well.
@@ -65,6 +69,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
             if (*abort_flag) return false;
             if (globaltimer_ns() - t0 > g_wait_limit_ns) {
                 *abort_flag = 1;
+                const uint64_t t1 = globaltimer_ns();
+                while (globaltimer_ns() - t1 < kLandingNs) {}
                 return false;
             }
         }
