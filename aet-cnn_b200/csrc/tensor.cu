@@ -421,6 +421,12 @@ void pinned_block_give(void *block) { pool_give(block); }
 // was taken into use has run.  A region is at most kRingHalf bytes: callers cut larger data into pieces.
 int ctx_ring(aet_context *ctx, size_t bytes, void **host) {
     bytes = round_up_sz(bytes, 256);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess) cudaGetLastError();
+    if (cap != cudaStreamCaptureStatusNone) {   // a replay would read (or fill) the region when it holds something else
+        aet_set_error("host data cannot be handed over while the context's stream is being captured");
+        return AET_E_CUDA;
+    }
     if (!ctx->ring && !(ctx->ring = static_cast<unsigned char *>(pool_take()))) {
         aet_set_error("page-locked staging memory could not be allocated");
         return AET_E_NOMEM;

@@ -271,3 +271,33 @@ def test_passes_that_keep_changing_are_not_captured_each_time(aet, ctx):
     assert median([lambda k=k: net.predict_topk(x, k) for k in (3, 4, 5)]) <= 1.7 * plain
     assert median([lambda: net.predict_topk(x, 3)]) <= 1.2 * plain
     net.close()
+
+
+def test_host_data_is_refused_while_the_stream_is_captured(aet):
+    """A captured upload would read its staging memory again at every replay, long after that holds something else."""
+    import torch
+    stream = torch.cuda.Stream()
+    ctx = aet.Context(0, stream=stream.cuda_stream)
+    net = cifar(aet, ctx, batch=2)
+    (x, t), = batches(net, 1)
+    for _ in range(2):
+        net.train(x, t)
+    layer = net.layer(0)
+    w, b = layer.read(aet.P_WEIGHTS), layer.read(aet.P_BIASES)
+    net.input.write(x)
+    net.truth.write(t)
+    ctx.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        for call in (lambda: net.input.write(x), lambda: layer.write(aet.P_WEIGHTS, w), lambda: layer.write(aet.P_BIASES, b), lambda: net.train(x, t),
+                     lambda: net.augment_input(x, [{}] * 2)):
+            with pytest.raises(aet.AetError, match="captured"):
+                call()
+        net.train_device(want_loss=False)
+    w = layer.read(aet.P_WEIGHTS)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert not np.array_equal(layer.read(aet.P_WEIGHTS), w)
+    del graph
+    net.close()
+    ctx.close()
