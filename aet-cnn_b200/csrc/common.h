@@ -508,8 +508,12 @@ struct StatusTap {
     int *host;
 };
 #ifdef __CUDACC__
-__device__ __forceinline__ void status_tap(const StatusTap &t) {   // behind pdl_enter: every kernel in front has ended
-    if (t.host && blockIdx.x + blockIdx.y + blockIdx.z + threadIdx.x == 0) *t.host = __ldcg(t.status);
+// Behind pdl_enter every kernel in front has ended: asked for with the kernel's other loads, stored with its results.
+__device__ __forceinline__ int status_ask(const StatusTap &t) {
+    return t.host && blockIdx.x + blockIdx.y + blockIdx.z + threadIdx.x == 0 ? __ldcg(t.status) : 0;
+}
+__device__ __forceinline__ void status_leave(const StatusTap &t, int status) {
+    if (t.host && blockIdx.x + blockIdx.y + blockIdx.z + threadIdx.x == 0) *t.host = status;
 }
 #endif
 int tensor_download_staged(aet_context *ctx, const float *dev_nhwc, float *out_nchw, int n, int c, int h, int w, int cp, StatusTap tap);

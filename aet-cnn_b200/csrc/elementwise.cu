@@ -1660,7 +1660,7 @@ constexpr int TOPK_WARPS = 4;
 __global__ void __launch_bounds__(TOPK_WARPS * 32)
 top_k_warp_kernel(const float *__restrict__ scores, int samples, int n, int ld, int k, int *__restrict__ index, StatusTap tap) {
     pdl_enter();
-    status_tap(tap);
+    const int status = status_ask(tap);
     const int s = blockIdx.x * TOPK_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (s >= samples) return;
     const float *a = scores + (size_t)s * ld;
@@ -1702,6 +1702,7 @@ top_k_warp_kernel(const float *__restrict__ scores, int samples, int n, int ld, 
         }
         if (plain) {
             if (lane < k) index[(size_t)s * k + lane] = mine;
+            status_leave(tap, status);
             return;
         }
     }
@@ -1741,11 +1742,12 @@ top_k_warp_kernel(const float *__restrict__ scores, int samples, int n, int ld, 
     }
     }
     if (lane < k) index[(size_t)s * k + lane] = id;
+    status_leave(tap, status);
 }
 // more slots than lanes: one thread per sample runs the loop as it stands
 __global__ void top_k_kernel(const float *__restrict__ scores, int samples, int n, int ld, int k, int *__restrict__ index, StatusTap tap) {
     pdl_enter();
-    status_tap(tap);
+    const int status = status_ask(tap);
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= samples) return;
     const float *a = scores + (size_t)s * ld;
@@ -1762,6 +1764,7 @@ __global__ void top_k_kernel(const float *__restrict__ scores, int samples, int 
             if (curr < 0) break;   // an empty slot was filled: the remaining slots are empty too and stay so
         }
     }
+    status_leave(tap, status);
 }
 
 struct ReducePlan {

@@ -40,7 +40,7 @@ template <bool TO_NHWC>
 __global__ void __launch_bounds__(kLayoutThreads)
 layout_pixel_kernel(const float *__restrict__ src, const float *__restrict__ add, float *__restrict__ dst, int n, int c, int hw, int cp, StatusTap tap) {
     pdl_enter();
-    if (!TO_NHWC) status_tap(tap);
+    const int status = TO_NHWC ? 0 : status_ask(tap);
     const size_t e = (size_t)blockIdx.x * kLayoutThreads + threadIdx.x;
     if (e >= (size_t)n * hw) return;
     const size_t b = e / hw, p = e - b * hw;
@@ -67,6 +67,7 @@ layout_pixel_kernel(const float *__restrict__ src, const float *__restrict__ add
             if (k + 2 < c) d[(size_t)(k + 2) * hw] = v.z;
             if (k + 3 < c) d[(size_t)(k + 3) * hw] = v.w;
         }
+        status_leave(tap, status);
     }
 }
 
@@ -75,7 +76,7 @@ template <bool TO_NHWC>
 __global__ void __launch_bounds__(kLayoutThreads)
 layout_block_kernel(const float *__restrict__ src, const float *__restrict__ add, float *__restrict__ dst, int c, int hw, int cp, StatusTap tap) {
     pdl_enter();
-    if (!TO_NHWC) status_tap(tap);
+    const int status = TO_NHWC ? 0 : status_ask(tap);
     extern __shared__ float tile[];
     const int pitch = hw | 1;
     const size_t dense = (size_t)blockIdx.x * c * hw, padded = (size_t)blockIdx.x * cp * hw;
@@ -101,6 +102,7 @@ layout_block_kernel(const float *__restrict__ src, const float *__restrict__ add
             const int ch = e / hw;
             dst[dense + e] = tile[ch * pitch + e - ch * hw];
         }
+        status_leave(tap, status);
     }
 }
 
@@ -109,7 +111,7 @@ template <bool TO_NHWC>
 __global__ void __launch_bounds__(kLayoutThreads)
 layout_tile_kernel(const float *__restrict__ src, const float *__restrict__ add, float *__restrict__ dst, int n, int c, int hw, int cp, StatusTap tap) {
     pdl_enter();
-    if (!TO_NHWC) status_tap(tap);
+    const int status = TO_NHWC ? 0 : status_ask(tap);
     __shared__ float tile[32][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int p0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
@@ -138,6 +140,7 @@ layout_tile_kernel(const float *__restrict__ src, const float *__restrict__ add,
         }
         __syncthreads();
     }
+    if (!TO_NHWC) status_leave(tap, status);
 }
 
 // Pieces of a staged upload, read by the SMs from page-locked host memory: a DMA transfer costs 8 us beside its bytes
