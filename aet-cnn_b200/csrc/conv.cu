@@ -881,10 +881,6 @@ static int conv_wgrad_one(aet_layer *l, const float *x, const float *dy, float *
             return launch_wgrad_reduce(ctx, tpartial, dw, out_floats, tsplits, accumulate);
         }
     }
-    {
-        const int r = igemm_wgrad(l, a, dw, accumulate, flops);
-        if (r != 1) return r;
-    }
     // N tile: the multiple of 16 (<= 256) that wastes the fewest padded columns, larger on ties
     int best_bn = 16, best_pad = 1 << 30;
     const int full = round_up(a.n_cols, 16);
@@ -905,6 +901,10 @@ static int conv_wgrad_one(aet_layer *l, const float *x, const float *dy, float *
     const int slabs_per_split = (total_slabs + want - 1) / want;
     const int splits = (total_slabs + slabs_per_split - 1) / slabs_per_split;
     a.k_per_split = slabs_per_split * BK;
+    {
+        const int r = igemm_wgrad(l, a, dw, accumulate, flops);
+        if (r != 1) return r;
+    }
     a.split_stride = (long long)out_floats;
     // One split that overwrites (a training step's first and only gradient of this layer): the tiles go straight to
     // their place, without the trip through scratch and the second kernel (a fully connected layer's gradient is as

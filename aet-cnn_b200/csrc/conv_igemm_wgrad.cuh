@@ -23,6 +23,7 @@ struct IgemmWgradArgs {
     float *out;
     int bn, filters, out_ld, dy_blocks;   // dy_blocks: copies per slab of the delta (0: one copy of all its 32-filter blocks)
     int m_tiles, n_tiles, splits, slabs, slabs_per_split;
+    int chunk_slabs;            // slabs summed in one accumulator
     long long split_stride;
     int stages, tmem_cols;
     uint32_t tx_bytes, b_bytes;
@@ -79,44 +80,54 @@ conv_wgrad_igemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
         return left < a.slabs_per_split ? (left > 0 ? left : 0) : a.slabs_per_split;
     };
 
+    const int step = X3 ? a.chunk_slabs : a.slabs_per_split;
+
     if (warp < 4) {
         // ------------------------------------------------------------------ epilogue: a warp's 32 lanes are one 32-channel block
         uint32_t tcount = 0;
-        for (int t = unit; t < total_tiles; t += units, ++tcount) {
+        bool ok = true;
+        for (int t = unit; t < total_tiles && ok; t += units) {
             const int sp = split_of(t), q = t - sp * per_split, nt = q / a.m_tiles, mt = q - nt * a.m_tiles;
-            const uint32_t b = tcount & 1u;
-            bool ok = mbar_wait(smem_u32(&ctl.acc_full[b]), (tcount >> 1) & 1u, abort_flag);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            tc_fence_after_sync();
             const int blk = mt * (PAIR ? 8 : 4) + (int)prank * 4 + warp;
             const int tap = blk / a.blocks_per_tap, c = (blk - tap * a.blocks_per_tap) * 32 + lane;
             const bool live = blk < a.blocks && c < a.cp;
             const int n0 = nt * a.bn;
             float *dst = a.out + (size_t)sp * a.split_stride + (size_t)n0 * a.out_ld + (size_t)tap * a.cp + c;
-            const bool have = slabs_of(sp) > 0;
-            const uint32_t src = tmem + b * (uint32_t)a.bn + ((uint32_t)(warp * 32) << 16);
-            for (int c0 = 0; c0 < a.bn; c0 += 32) {
-                uint32_t v[32];
-                if (have) {
-                    tmem_ld16_issue(src + (uint32_t)c0, v);
-                    tmem_ld16_issue(src + (uint32_t)c0 + 16u, v + 16);
-                    tmem_ld_wait();
-                } else {
+            const int slabs = slabs_of(sp);
+            const bool have = slabs > 0;
+            for (int k0 = 0; k0 == 0 || k0 < slabs; k0 += step, ++tcount) {
+                const uint32_t b = tcount & 1u;
+                ok = mbar_wait(smem_u32(&ctl.acc_full[b]), (tcount >> 1) & 1u, abort_flag);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                tc_fence_after_sync();
+                const uint32_t src = tmem + b * (uint32_t)a.bn + ((uint32_t)(warp * 32) << 16);
+                for (int c0 = 0; c0 < a.bn; c0 += 32) {
+                    uint32_t v[32];
+                    if (have) {
+                        tmem_ld16_issue(src + (uint32_t)c0, v);
+                        tmem_ld16_issue(src + (uint32_t)c0 + 16u, v + 16);
+                        tmem_ld_wait();
+                    } else {
 #pragma unroll
-                    for (int k = 0; k < 32; ++k) v[k] = 0u;
-                }
-                if (live) {
+                        for (int k = 0; k < 32; ++k) v[k] = 0u;
+                    }
+                    if (X3 && k0 > 0) {   // added where the sum is, by this thread alone and in order: nothing to wait for
 #pragma unroll
-                    for (int k = 0; k < 32; ++k)
-                        if (n0 + c0 + k < a.filters) dst[(size_t)(c0 + k) * a.out_ld] = __uint_as_float(v[k]);
+                        for (int k = 0; k < 32; ++k)
+                            if (live && n0 + c0 + k < a.filters) atomicAdd(dst + (size_t)(c0 + k) * a.out_ld, __uint_as_float(v[k]));
+                    } else if (live) {
+#pragma unroll
+                        for (int k = 0; k < 32; ++k)
+                            if (n0 + c0 + k < a.filters) dst[(size_t)(c0 + k) * a.out_ld] = __uint_as_float(v[k]);
+                    }
                 }
-            }
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) {
-                if (PAIR) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl.acc_empty[b]), 0));
-                else mbar_arrive(smem_u32(&ctl.acc_empty[b]));
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) {
+                    if (PAIR) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl.acc_empty[b]), 0));
+                    else mbar_arrive(smem_u32(&ctl.acc_empty[b]));
+                }
             }
         }
     } else if (warp == 4) {
@@ -129,42 +140,45 @@ conv_wgrad_igemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
             const uint32_t wait0 = smem_u32(X3 ? &ctl.ready[0] : &ctl.full[0]), empty0 = smem_u32(&ctl.empty[0]);
             uint32_t s = 0, phase = 0, tcount = 0;
             bool ok = true;
-            for (int t = unit; t < total_tiles && ok; t += units, ++tcount) {
+            for (int t = unit; t < total_tiles && ok; t += units) {
                 const int slabs = slabs_of(split_of(t));
-                const uint32_t b = tcount & 1u, d = tmem + b * (uint32_t)a.bn;
-                if (!mbar_wait(smem_u32(&ctl.acc_empty[b]), ((tcount >> 1) & 1u) ^ 1u, abort_flag)) break;
-                tc_fence_after_sync();
-                uint32_t accumulate = 0;
-                for (int k = 0; k < slabs; ++k) {
-                    ok = mbar_wait(wait0 + s * 8u, phase, abort_flag);
-                    if (!ok) break;
+                for (int k0 = 0; ok && (k0 == 0 || k0 < slabs); k0 += step, ++tcount) {
+                    const int k1 = slabs - k0 < step ? slabs : k0 + step;
+                    const uint32_t b = tcount & 1u, d = tmem + b * (uint32_t)a.bn;
+                    if (!mbar_wait(smem_u32(&ctl.acc_empty[b]), ((tcount >> 1) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
                     tc_fence_after_sync();
-                    const uint32_t st16 = (s * stage_bytes) >> 4;
+                    uint32_t accumulate = 0;
+                    for (int k = k0; k < k1; ++k) {
+                        ok = mbar_wait(wait0 + s * 8u, phase, abort_flag);
+                        if (!ok) break;
+                        tc_fence_after_sync();
+                        const uint32_t st16 = (s * stage_bytes) >> 4;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const uint64_t ah = da0 + st16 + (uint64_t)(j * 64), bh = db0 + st16 + (uint64_t)(j * 64);
-                        const uint32_t first = j > 0 ? 1u : accumulate;
-                        if (X3) {
-                            if (PAIR) {
-                                mma_tf32_pair(d, ah + lo16, bh, idesc, first);
-                                mma_tf32_pair(d, ah, bh + lo16, idesc, 1u);
-                                mma_tf32_pair(d, ah, bh, idesc, 1u);
-                            } else {
-                                mma_tf32(d, ah + lo16, bh, idesc, first);
-                                mma_tf32(d, ah, bh + lo16, idesc, 1u);
-                                mma_tf32(d, ah, bh, idesc, 1u);
-                            }
-                        } else if (PAIR) mma_tf32_pair(d, ah, bh, idesc, first);
-                        else mma_tf32(d, ah, bh, idesc, first);
+                        for (int j = 0; j < 4; ++j) {
+                            const uint64_t ah = da0 + st16 + (uint64_t)(j * 64), bh = db0 + st16 + (uint64_t)(j * 64);
+                            const uint32_t first = j > 0 ? 1u : accumulate;
+                            if (X3) {
+                                if (PAIR) {
+                                    mma_tf32_pair(d, ah + lo16, bh, idesc, first);
+                                    mma_tf32_pair(d, ah, bh + lo16, idesc, 1u);
+                                    mma_tf32_pair(d, ah, bh, idesc, 1u);
+                                } else {
+                                    mma_tf32(d, ah + lo16, bh, idesc, first);
+                                    mma_tf32(d, ah, bh + lo16, idesc, 1u);
+                                    mma_tf32(d, ah, bh, idesc, 1u);
+                                }
+                            } else if (PAIR) mma_tf32_pair(d, ah, bh, idesc, first);
+                            else mma_tf32(d, ah, bh, idesc, first);
+                        }
+                        accumulate = 1u;
+                        if (PAIR) mma_commit_pair(empty0 + s * 8u, 3);
+                        else mma_commit(empty0 + s * 8u);
+                        if (++s == (uint32_t)a.stages) { s = 0; phase ^= 1u; }
                     }
-                    accumulate = 1u;
-                    if (PAIR) mma_commit_pair(empty0 + s * 8u, 3);
-                    else mma_commit(empty0 + s * 8u);
-                    if (++s == (uint32_t)a.stages) { s = 0; phase ^= 1u; }
+                    if (!ok) break;
+                    if (PAIR) mma_commit_pair(smem_u32(&ctl.acc_full[b]), 3);
+                    else mma_commit(smem_u32(&ctl.acc_full[b]));
                 }
-                if (!ok) break;
-                if (PAIR) mma_commit_pair(smem_u32(&ctl.acc_full[b]), 3);
-                else mma_commit(smem_u32(&ctl.acc_full[b]));
             }
         }
     } else if (warp < 8) {
@@ -345,6 +359,13 @@ int igemm_wgrad(aet_layer *l, const ConvArgs &ca, float *dw, int accumulate, dou
     t.m_tiles = (blocks + (plan.pair ? 7 : 3)) / (plan.pair ? 8 : 4); t.n_tiles = (g.K + plan.bn - 1) / plan.bn;
     t.slabs = slabs; t.slabs_per_split = (slabs + plan.splits - 1) / plan.splits;
     t.splits = (slabs + t.slabs_per_split - 1) / t.slabs_per_split;
+    // 3xTF32: the tensor core truncates its running sums, so an error of the accumulator grows with their length (5e-6 and more
+    // over a few hundred slabs, where rounding costs 1e-6).  No accumulator sums more slabs here than the gather kernel's
+    // split of the same layer; longer splits go in equal chunks, which the epilogue adds up in memory (round to nearest)
+    // beside the next one's MMAs.  64 -> 128 filters on 16x16 maps, batch 128: chunks of 11 slabs.  A training step of that
+    // network takes 496 us instead of 491, and errs by no more than the gather kernel.
+    const int longest = ca.k_per_split / BK, chunks = (t.slabs_per_split + longest - 1) / longest;
+    t.chunk_slabs = (t.slabs_per_split + chunks - 1) / chunks;
     t.split_stride = (long long)out_floats;
     const bool direct = t.splits == 1 && !accumulate;
     t.out = dw;

@@ -60,6 +60,44 @@ def test_conv_im2col(aet, ctx, oracle, oracle64, shape, math):
         assert any(n.startswith(want) and (not n.startswith("conv_%s_tma.i2c_" % kind) or ("_x3" in n) == x3) for n in names), (want, names)
 
 
+@pytest.mark.parametrize("shape", [
+    (17, 36, 28, 19, 40, 5, 1, 2),      # 289 slabs of pixels: the gather kernel sums five in an accumulator
+    (33, 72, 29, 30, 64, 1, 1, 0),
+    (33, 48, 17, 10, 4, 5, 1, 2),       # four filters
+    (64, 64, 16, 16, 128, 3, 1, 1),     # filters by two, a pair of CTAs
+])
+def test_weight_gradient_in_3xtf32_sums_no_more_at_a_time_than_the_gather_kernel(aet, ctx, shape):
+    """Both kernels against float64.  The error is that of the tensor core's running sums, so it grows with what one
+    accumulator takes; over the 500 and more weights here its norm varies by a few per cent."""
+    import torch
+    n, c, h, w, k, size, stride, pad = shape
+    rng = np.random.default_rng(h * w)
+    x = rng.standard_normal((n, c, h, w)).astype(np.float32)
+    dy = rng.standard_normal((n, k, (h + 2 * pad - size) // stride + 1, (w + 2 * pad - size) // stride + 1)).astype(np.float32)
+    ref = torch.nn.grad.conv2d_weight(torch.from_numpy(x).double(), (k, c, size, size), torch.from_numpy(dy).double(), stride, pad).numpy()
+    err = {}
+    ctx.set_math(aet.MATH_3XTF32)
+    try:
+        for gather in (0, 1):
+            ctx.set_option("gather_only", gather)
+            layer = aet.ConvolutionalLayer(ctx, n, h, w, c, k, size, stride, stride, pad, aet.LINEAR, 0, 1)
+            xin = aet.Tensor(ctx, n, c, h, w)
+            xin.write(x)
+            layer.write(aet.P_DELTA, dy)
+            ctx.profile(1)
+            layer.backward(aet.make_state(input=xin, train=1))
+            assert any(v.startswith("conv_wgrad_gather" if gather else "conv_wgrad_tma.i2c_") for v in variants_used(ctx))
+            ctx.profile(0)
+            err[gather] = rel_l2(layer.read(aet.P_WEIGHT_UPDATES), ref)
+            layer.close()
+            xin.close()
+    finally:
+        ctx.profile(0)
+        ctx.set_option("gather_only", 0)
+        ctx.set_math(aet.MATH_TF32)
+    assert err[0] <= 1.1 * err[1] <= TOL_3X, err
+
+
 @pytest.mark.parametrize("batch", [1, 2, 3, 4, 5])
 @pytest.mark.parametrize("inputs,filters", [(64, 10), (4100, 37), (9216, 512)])
 def test_fully_connected_of_few_images(aet, ctx, oracle, batch, inputs, filters):
