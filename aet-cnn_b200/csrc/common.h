@@ -127,6 +127,7 @@ struct aet_context {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_gram = nullptr;   // ev_gram: the Gram matrix of this pass's input patches is there
     bool overlap_wgrad = false;   // set by the network around its backward pass
     bool wgrad_fresh = false;     // set by a training step without subdivisions: the gradient arena is zero when backward starts, the weight gradients may overwrite
+    aet_network *update_in = nullptr;   // set by a training step whose update follows at once: weight gradients may apply it themselves
     bool on_side = false, side_pending = false;
     float *scratch_side = nullptr;
     size_t scratch_side_bytes = 0;
@@ -200,6 +201,8 @@ struct aet_layer {
     ParamArena *arena = nullptr;
     ParamArena own_arena;
     ParamSegment seg_w, seg_b, seg_s;
+    int seg_id = 0;                      // of the weights, in the network's update tables
+    bool updated = false;                // this pass's weight gradient has applied the update to the weights already
     float *mean = nullptr, *variance = nullptr, *rolling_mean = nullptr, *rolling_variance = nullptr;
     float *inv_std = nullptr;            // per-channel 1/std in the parity mode's form
     float *bwd_coef = nullptr;           // [3][ocp] coefficients of the BN backward apply pass
@@ -543,6 +546,10 @@ struct ConvStats {
 int conv_fprop(aet_layer *l, const float *x, float *y, const float *bias, int act_in_epilogue, ConvStats *stats = nullptr);
 int conv_dgrad(aet_layer *l, const float *dy, float *dx);
 int conv_wgrad(aet_layer *l, const float *x, const float *dy, float *dw, int accumulate);
+// The weight gradient can apply the step's update in its epilogue (then it has to run behind the data gradient, which reads
+// the weights); conv_wgrad_update runs it and marks the layer as updated.
+bool conv_update_ok(const aet_layer *l);
+int conv_wgrad_update(aet_layer *l, const float *x, const float *dy);
 void conv_release(aet_layer *l);
 
 int k_bn_stats(aet_layer *l, int update_rolling, const ConvStats *from_epilogue = nullptr);
@@ -591,6 +598,7 @@ void pinned_block_give(void *block);
 int k_param_hash(aet_context *ctx, const float *p, size_t count, uint64_t *hash_dev);
 int k_augment(aet_context *ctx, const float *src_nchw, int n, int c, int sh, int sw, float *dst_nhwc, int size, int cp,
               const aet_augment *params_dev);
+constexpr int kMaxUpdated = 8;   // most layers of a network that update themselves in one pass
 constexpr int kTopkLanes = 32;   // lists of up to this many entries are held by a warp's lanes
 int k_top_k(aet_context *ctx, const float *scores, int samples, int n, int ld, int k, int *index_dev, StatusTap tap = {});
 

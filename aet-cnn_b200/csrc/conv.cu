@@ -22,6 +22,8 @@
 // warp 4 allocates TMEM and its lane 0 issues every MMA.
 #include "common.h"
 #include "umma.cuh"
+#include "sgd_update.cuh"
+#include <float.h>
 #include "activation.cuh"
 #include <cooperative_groups.h>
 #include <deque>
@@ -928,6 +930,21 @@ int conv_wgrad(aet_layer *l, const float *x, const float *dy, float *dw, int acc
         if (r != 1) return r;
     }
     for (int gi = 0; gi < l->groups; ++gi) AET_TRY(conv_wgrad_one(l, x, dy, dw, accumulate, gi));
+    return AET_OK;
+}
+
+bool conv_update_ok(const aet_layer *l) {
+    const aet_network *net = l->ctx->update_in;
+    if (!net || l->net != net || l->arena != &net->arena) return false;
+    int updated = 0;
+    for (const aet_layer *q : net->layers) updated += q->updated;
+    return updated < kMaxUpdated && igemm_update_ok(l, layer_geom(l));
+}
+
+int conv_wgrad_update(aet_layer *l, const float *x, const float *dy) {
+    const ConvGeom g = layer_geom(l);
+    AET_TRY(igemm_wgrad_update(l, g, x, dy, 2.0 * g.N * (double)g.K * g.C));
+    l->updated = true;
     return AET_OK;
 }
 

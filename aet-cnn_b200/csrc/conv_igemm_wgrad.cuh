@@ -27,12 +27,44 @@ struct IgemmWgradArgs {
     long long split_stride;
     int stages, tmem_cols;
     uint32_t tx_bytes, b_bytes;
+    float *W, *U;               // UPDATE: the weights and their momentum, laid out like `out`
+    const float *seg, *hyper;   // ... and the step's constants (see sgd_step)
     int *status;
     unsigned long long *span;
 };
 
-template <bool PAIR, bool X3>
-__global__ void __launch_bounds__(256 + (X3 ? IG_CONVERTERS * 32 : 0), 1)
+constexpr int IG_UPDATERS = 12;   // UPDATE: epilogue warps, three to a quarter of the lanes
+
+// 32 channels (the lanes) of 16 filters, `off` bytes into the segment and `ld` bytes from one filter to the next: all loads are
+// in flight before the first is used.  FULL: all 16 filters exist.
+template <bool FULL>
+__device__ __forceinline__ bool update_rows(float *W, float *U, uint32_t off, uint32_t ld, int rows, const uint32_t (&g)[16], const SgdStep &s) {
+    char *wb = reinterpret_cast<char *>(W), *ub = reinterpret_cast<char *>(U);
+    float w[16], u[16];
+    bool hit = false;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        if (!FULL && k >= rows) break;
+        w[k] = __ldcs(reinterpret_cast<const float *>(wb + (off + k * ld)));
+        u[k] = __ldcs(reinterpret_cast<const float *>(ub + (off + k * ld)));
+    }
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        if (!FULL && k >= rows) break;
+        u[k] += __uint_as_float(g[k]);
+        if (!s.frozen) {
+            // one addition tells whether both are finite (or large enough for a closer look)
+            if (s.scrub && !(fabsf(u[k]) + fabsf(w[k]) <= FLT_MAX)) hit |= scrub1(w[k], u[k], s.scrub, (off + k * ld) / 4);
+            sgd_move(w[k], u[k], s.rate, s.momentum, s.decay);
+            __stcs(reinterpret_cast<float *>(wb + (off + k * ld)), w[k]);
+        }
+        __stcs(reinterpret_cast<float *>(ub + (off + k * ld)), u[k]);
+    }
+    return hit;
+}
+
+template <bool PAIR, bool X3, bool UPDATE>
+__global__ void __launch_bounds__(256 + (X3 ? IG_CONVERTERS * 32 : (UPDATE ? (IG_UPDATERS - 4) * 32 : 0)), 1)
 conv_wgrad_igemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_dy, const IgemmWgradArgs a) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ IgemmCtl ctl;
@@ -54,7 +86,7 @@ conv_wgrad_igemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&ctl.acc_full[b]), 1);
-            mbar_init(smem_u32(&ctl.acc_empty[b]), PAIR ? 8 : 4);
+            mbar_init(smem_u32(&ctl.acc_empty[b]), UPDATE ? IG_UPDATERS : (PAIR ? 8 : 4));
         }
         ctl.abort_flag = 0;
         fence_barrier_init();
@@ -82,7 +114,41 @@ conv_wgrad_igemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
 
     const int step = X3 ? a.chunk_slabs : a.slabs_per_split;
 
-    if (warp < 4) {
+    if (UPDATE && (warp < 4 || warp >= 8)) {
+        // ------------------------------------------------------------------ epilogue that updates the weights (warps 0-3, 8-15)
+        const int quarter = warp & 3, share = warp < 4 ? 0 : (warp - 4) >> 2;   // this warp's lanes, and which 16 of 48 filters
+        const SgdStep s = sgd_step(a.seg, a.hyper);
+        const uint32_t ld = (uint32_t)a.out_ld * 4u;
+        bool hit = false;
+        uint32_t tcount = 0;
+        for (int t = unit; t < total_tiles; t += units, ++tcount) {
+            const int nt = t / a.m_tiles, mt = t - nt * a.m_tiles;
+            const int blk = mt * 4 + quarter, tap = blk / a.blocks_per_tap, c = (blk - tap * a.blocks_per_tap) * 32 + lane;
+            const bool live = blk < a.blocks && c < a.cp;
+            const int n0 = nt * a.bn;
+            const uint32_t b = tcount & 1u;
+            bool ok = mbar_wait(smem_u32(&ctl.acc_full[b]), (tcount >> 1) & 1u, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after_sync();
+            const uint32_t src = tmem + b * (uint32_t)a.bn + ((uint32_t)(quarter * 32) << 16);
+            for (int c0 = share * 16; c0 < a.bn; c0 += IG_UPDATERS * 4) {
+                __syncwarp();
+                uint32_t v[16];
+                tmem_ld16_issue(src + (uint32_t)c0, v);
+                tmem_ld_wait();
+                const int rows = a.filters - n0 - c0;
+                const uint32_t off = (uint32_t)(n0 + c0) * ld + (uint32_t)(tap * a.cp + c) * 4u;
+                if (!live || rows <= 0) continue;
+                if (rows >= 16) hit |= update_rows<true>(a.W, a.U, off, ld, 16, v, s);
+                else hit |= update_rows<false>(a.W, a.U, off, ld, rows, v, s);
+            }
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&ctl.acc_empty[b]));
+        }
+        if (hit && a.status) atomicOr(a.status, AET_STATUS_NAN);
+    } else if (warp < 4) {
         // ------------------------------------------------------------------ epilogue: a warp's 32 lanes are one 32-channel block
         uint32_t tcount = 0;
         bool ok = true;
@@ -301,7 +367,7 @@ IgemmPlan igemm_wgrad_plan(const aet_context *ctx, int blocks, int filters, int 
     return best;
 }
 
-template <bool PAIR, bool X3>
+template <bool PAIR, bool X3, bool UPDATE = false>
 int igemm_wgrad_launch(aet_context *ctx, const CUtensorMap &mx, const CUtensorMap &mdy, IgemmWgradArgs &a, const char *variant, double flops) {
     a.b_bytes = (uint32_t)(PAIR ? a.bn / 2 : a.bn) * BK * 4;
     a.tx_bytes = (uint32_t)BM * BK * 4 + a.b_bytes;
@@ -312,14 +378,50 @@ int igemm_wgrad_launch(aet_context *ctx, const CUtensorMap &mx, const CUtensorMa
     a.tmem_cols = pow2_cols(2 * a.bn);
     a.status = ctx->status_dev;
     const size_t smem_bytes = stage * stages + 1024;
-    AET_TRY(ctx_smem_attr(ctx, conv_wgrad_igemm_kernel<PAIR, X3>));
+    AET_TRY(ctx_smem_attr(ctx, conv_wgrad_igemm_kernel<PAIR, X3, UPDATE>));
     const int tiles = a.m_tiles * a.n_tiles * a.splits, units = PAIR ? ctx->sm_count / 2 : ctx->sm_count;
     const int grid = (tiles < units ? tiles : units) * (PAIR ? 2 : 1);
     LaunchScope scope(ctx, "conv_wgrad_tma", 0, flops, variant);
     a.span = ctx->span_ptr;
-    if (PAIR) launch_k_cluster(ctx->stream, dim3(grid), dim3(256 + (X3 ? IG_CONVERTERS * 32 : 0)), smem_bytes, 2, 1, conv_wgrad_igemm_kernel<PAIR, X3>, mx, mdy, a);
-    else launch_k(ctx->stream, dim3(grid), dim3(256 + (X3 ? IG_CONVERTERS * 32 : 0)), smem_bytes, conv_wgrad_igemm_kernel<PAIR, X3>, mx, mdy, a);
+    if (PAIR) launch_k_cluster(ctx->stream, dim3(grid), dim3(256 + (X3 ? IG_CONVERTERS * 32 : (UPDATE ? (IG_UPDATERS - 4) * 32 : 0))), smem_bytes, 2, 1, conv_wgrad_igemm_kernel<PAIR, X3, UPDATE>, mx, mdy, a);
+    else launch_k(ctx->stream, dim3(grid), dim3(256 + (X3 ? IG_CONVERTERS * 32 : (UPDATE ? (IG_UPDATERS - 4) * 32 : 0))), smem_bytes, conv_wgrad_igemm_kernel<PAIR, X3, UPDATE>, mx, mdy, a);
     return aet_check_launch("conv_wgrad_tma");
+}
+
+// What the launchers have in common, the geometry and the copies' maps for a plan; 1 = not eligible.
+bool igemm_wgrad_ok(const aet_layer *l, const ConvGeom &g, Im2colBox &box) {
+    const int p = g.pad * g.dil, ext_w = (g.S - 1) * g.dil, ext_h = (g.R - 1) * g.dil;
+    box = {-p, -p, p - ext_w, p - ext_h, g.sx, BK};
+    return igemm_common_ok(l, g) && im2col_ok(g.xs, g.W, g.H, g.N, box, g.R, g.dil) && (g.W + 2 * p - ext_w - 1) / g.sx + 1 == g.OW &&
+           (g.H + 2 * p - ext_h - 1) / g.sy + 1 == g.OH;
+}
+int igemm_wgrad_setup(aet_layer *l, const ConvGeom &g, const float *x, const float *dy, const Im2colBox &box, const IgemmPlan &plan,
+                      IgemmWgradArgs &t, CUtensorMap *mx, const CUtensorMap **mdy) {
+    const int p = g.pad * g.dil, per_tap = (g.cp + 31) / 32, pixels = g.N * g.OH * g.OW;
+    const int bnc = plan.pair ? plan.bn / 2 : plan.bn;
+    AET_TRY(get_map_im2col(l, 29, x, g.cp, g.xs, g.W, g.H, g.N, box, true, mx));
+    if (g.kp % 32 == 0) {
+        cuuint64_t dims[3] = {32, (cuuint64_t)pixels, (cuuint64_t)g.kp / 32};
+        cuuint64_t str[2] = {(cuuint64_t)g.ys * 4, 128};
+        cuuint32_t bx[3] = {32, BK, (cuuint32_t)bnc / 32};
+        AET_TRY(get_map(l, 30, dy, 3, dims, str, bx, true, mdy));
+    } else {
+        cuuint64_t dims[2] = {(cuuint64_t)g.kp, (cuuint64_t)pixels};
+        cuuint64_t str[1] = {(cuuint64_t)g.ys * 4};
+        cuuint32_t bx[2] = {32, BK};
+        AET_TRY(get_map(l, 31, dy, 2, dims, str, bx, true, mdy));
+        t.dy_blocks = bnc / 32;
+    }
+    t.hw = g.OH * g.OW; t.w = g.OW; t.div_hw = make_fastdiv(t.hw); t.div_w = make_fastdiv(t.w);
+    t.step = g.sx; t.h0 = t.w0 = -p; t.dil = g.dil; t.S = g.S;
+    t.cp = g.cp; t.blocks_per_tap = per_tap; t.blocks = g.R * g.S * per_tap;
+    t.bn = plan.bn; t.filters = g.K; t.out_ld = g.R * g.S * g.cp;
+    t.m_tiles = (t.blocks + (plan.pair ? 7 : 3)) / (plan.pair ? 8 : 4); t.n_tiles = (g.K + plan.bn - 1) / plan.bn;
+    t.slabs = (pixels + BK - 1) / BK;
+    t.slabs_per_split = (t.slabs + plan.splits - 1) / plan.splits;
+    t.splits = (t.slabs + t.slabs_per_split - 1) / t.slabs_per_split;
+    t.chunk_slabs = t.slabs_per_split;
+    return AET_OK;
 }
 
 // 1 = not eligible
@@ -327,38 +429,15 @@ int igemm_wgrad(aet_layer *l, const ConvArgs &ca, float *dw, int accumulate, dou
     const ConvGeom &g = ca.g;
     aet_context *ctx = l->ctx;
     const bool x3 = ctx->math == AET_MATH_3XTF32;
-    if (!igemm_common_ok(l, g)) return 1;
-    const int p = g.pad * g.dil, ext_w = (g.S - 1) * g.dil, ext_h = (g.R - 1) * g.dil;
-    const Im2colBox box = {-p, -p, p - ext_w, p - ext_h, g.sx, BK};
-    if (!im2col_ok(g.xs, g.W, g.H, g.N, box, g.R, g.dil)) return 1;
-    if ((g.W + 2 * p - ext_w - 1) / g.sx + 1 != g.OW || (g.H + 2 * p - ext_h - 1) / g.sy + 1 != g.OH) return 1;
-    const int per_tap = (g.cp + 31) / 32, blocks = g.R * g.S * per_tap, slabs = (ca.k_total + BK - 1) / BK;
+    Im2colBox box;
+    if (!igemm_wgrad_ok(l, g, box)) return 1;
+    const int blocks = g.R * g.S * ((g.cp + 31) / 32), slabs = (ca.k_total + BK - 1) / BK;
     const size_t out_floats = (size_t)g.K * ca.n_cols;
     const IgemmPlan plan = igemm_wgrad_plan(ctx, blocks, g.K, slabs, (double)out_floats, x3, !accumulate);
-    const int bnc = plan.pair ? plan.bn / 2 : plan.bn;
     IgemmWgradArgs t = {};
     CUtensorMap mx;
     const CUtensorMap *mdy;
-    AET_TRY(get_map_im2col(l, 29, ca.src_b, g.cp, g.xs, g.W, g.H, g.N, box, true, &mx));
-    if (g.kp % 32 == 0) {
-        cuuint64_t dims[3] = {32, (cuuint64_t)ca.k_total, (cuuint64_t)g.kp / 32};
-        cuuint64_t str[2] = {(cuuint64_t)g.ys * 4, 128};
-        cuuint32_t bx[3] = {32, BK, (cuuint32_t)bnc / 32};
-        AET_TRY(get_map(l, 30, ca.src_a, 3, dims, str, bx, true, &mdy));
-    } else {
-        cuuint64_t dims[2] = {(cuuint64_t)g.kp, (cuuint64_t)ca.k_total};
-        cuuint64_t str[1] = {(cuuint64_t)g.ys * 4};
-        cuuint32_t bx[2] = {32, BK};
-        AET_TRY(get_map(l, 31, ca.src_a, 2, dims, str, bx, true, &mdy));
-        t.dy_blocks = bnc / 32;
-    }
-    t.hw = g.OH * g.OW; t.w = g.OW; t.div_hw = make_fastdiv(t.hw); t.div_w = make_fastdiv(t.w);
-    t.step = g.sx; t.h0 = t.w0 = -p; t.dil = g.dil; t.S = g.S;
-    t.cp = g.cp; t.blocks_per_tap = per_tap; t.blocks = blocks;
-    t.bn = plan.bn; t.filters = g.K; t.out_ld = ca.out_ld;
-    t.m_tiles = (blocks + (plan.pair ? 7 : 3)) / (plan.pair ? 8 : 4); t.n_tiles = (g.K + plan.bn - 1) / plan.bn;
-    t.slabs = slabs; t.slabs_per_split = (slabs + plan.splits - 1) / plan.splits;
-    t.splits = (slabs + t.slabs_per_split - 1) / t.slabs_per_split;
+    AET_TRY(igemm_wgrad_setup(l, g, ca.src_b, ca.src_a, box, plan, t, &mx, &mdy));
     // 3xTF32: the tensor core truncates its running sums, so an error of the accumulator grows with their length (5e-6 and more
     // over a few hundred slabs, where rounding costs 1e-6).  No accumulator sums more slabs here than the gather kernel's
     // split of the same layer; longer splits go in equal chunks, which the epilogue adds up in memory (round to nearest)
@@ -379,6 +458,39 @@ int igemm_wgrad(aet_layer *l, const ConvArgs &ca, float *dw, int accumulate, dou
     else r = igemm_wgrad_launch<false, false>(ctx, mx, *mdy, t, variant, flops);
     if (r != AET_OK || direct) return r;
     return launch_wgrad_reduce(ctx, partial, dw, out_floats, t.splits, accumulate);
+}
+
+// Fully connected layers in a training step: the weight gradient's epilogue applies the update.  A gradient as large as the
+// weights, from a batch that is a few K slabs, is bound by memory: written, read again and cleared by the update it costs
+// 28 bytes per weight (4096 x 9216 at batch 128: 100 us alone and 157 of the update's 255), in the epilogue the 16 that the
+// weights and their momentum take (164 us; a step of the 227x227 network 2.31 -> 2.17 ms).  From a million weights on and up to
+// 8 slabs (256 images); below that, or where K is longer, the launch and the products count.  Offsets are 32 bits of bytes.
+bool igemm_update_ok(const aet_layer *l, const ConvGeom &g) {
+    Im2colBox box;
+    return l->ctx->math == AET_MATH_TF32 && l->groups == 1 && g.OH == 1 && g.OW == 1 && g.R == 1 && g.S == 1 && g.N <= 8 * BK &&
+           (double)g.K * g.cp >= 1048576.0 && (double)g.K * g.cp < 1073741824.0 && igemm_wgrad_ok(l, g, box);
+}
+int igemm_wgrad_update(aet_layer *l, const ConvGeom &g, const float *x, const float *dy, double flops) {
+    aet_context *ctx = l->ctx;
+    Im2colBox box;
+    if (!igemm_wgrad_ok(l, g, box)) { aet_set_error("internal: layer cannot update itself"); return AET_E_INVALID; }
+    // tiles of the width whose last round wastes least (a tile's cost: its columns, and 16 for its start)
+    IgemmPlan plan = {false, 256, 1, 0, 1};
+    const int mt = ((g.cp + 31) / 32 + 3) / 4;
+    int best = INT_MAX;
+    for (int bn = 256; bn >= 96; bn -= 32) {
+        const int rounds = (mt * ((g.K + bn - 1) / bn) + ctx->sm_count - 1) / ctx->sm_count;
+        if (rounds * (bn + 16) < best) { best = rounds * (bn + 16); plan.bn = bn; }
+    }
+    IgemmWgradArgs t = {};
+    CUtensorMap mx;
+    const CUtensorMap *mdy;
+    AET_TRY(igemm_wgrad_setup(l, g, x, dy, box, plan, t, &mx, &mdy));
+    const aet_network *net = ctx->update_in;
+    t.W = layer_W(l); t.U = layer_U(l); t.seg = net->seg_table + 4 * l->seg_id; t.hyper = net->hyper_dev;
+    char variant[32];
+    snprintf(variant, sizeof(variant), "i2c_n%d_sgd", plan.bn);
+    return igemm_wgrad_launch<false, false, true>(ctx, mx, *mdy, t, variant, flops);
 }
 
 }  // namespace

@@ -24,6 +24,7 @@
 #include "common.h"
 #include <climits>
 #include "activation.cuh"
+#include "sgd_update.cuh"
 
 namespace {
 
@@ -1402,21 +1403,6 @@ __global__ void __launch_bounds__(1024) tail_publish_kernel(const float *G, cons
 // Limit of the peer-flag wait below (nanoseconds); set per device by elementwise_set_wait_limit.
 __constant__ unsigned long long g_flag_wait_limit_ns = 1000000000ull;
 
-// Non-finite scrub of the reference's GPU update.  kind 1 = a weight segment: a NaN/Inf pending update becomes 0
-// (resetNanAndInf) and a NaN/Inf weight becomes 1 / (index + 1) (fixNanAndInf), mtcs/MtcsConvLayer.c:586-587,
-// mtcs/MtcsTool.c:77-107.  kind 2 = a bias / scale segment of a batch-norm layer with try_fix_nan: the pending
-// update becomes 1 / (index + 1), dnn/NLayer.c:318-323.  `index` is the element's position in its segment.
-// Returns true when something was replaced.
-__device__ __forceinline__ bool scrub1(float &w, float &u, int kind, size_t index) {
-    bool hit = false;
-    if (kind == 1) {
-        if (isnan(u) || isinf(u)) { u = 0.f; hit = true; }
-        if (isnan(w) || isinf(w)) { w = 1.0f / ((float)index + 1.f); hit = true; }
-    } else if (kind == 2) {
-        if (isnan(u) || isinf(u)) { u = 1.0f / ((float)index + 1.f); hit = true; }
-    }
-    return hit;
-}
 __device__ __forceinline__ bool scrub4(float4 &w, float4 &u, int kind, size_t index) {
     bool hit = scrub1(w.x, u.x, kind, index);
     hit |= scrub1(w.y, u.y, kind, index + 1);
@@ -1453,19 +1439,23 @@ __global__ void tail_wait_kernel(const TailArgs t) {
     }
 }
 
+// Arena blocks (1024 floats) that the pass has updated already: layers whose weight gradient applied its own update.
+struct UpdatedBlocks {
+    int ranges;
+    int first[kMaxUpdated], count[kMaxUpdated];   // ascending
+};
+
 // seg_table: four floats per segment {learning-rate multiplier, decay flag, scrub kind, first block (int bits)}
-__global__ void __launch_bounds__(TB) sgd_arena_kernel(float *W, float *U, float *G, const int *block_seg,
-                                                       const float *seg_table, const float *hyper, const TailArgs t, int *status) {
+__global__ void __launch_bounds__(TB) sgd_arena_kernel(float *W, float *U, float *G, const int *block_seg, const float *seg_table,
+                                                       const float *hyper, const UpdatedBlocks done, const TailArgs t, int *status) {
     pdl_enter();
-    const int seg = block_seg[blockIdx.x];
-    const bool frozen = seg_table[4 * seg] < 0.f;   // not updated now: the gradient joins the pending update, nothing else moves
-    const float rate = hyper[0] * seg_table[4 * seg];
-    const float momentum = hyper[1];
-    const float decay_term = seg_table[4 * seg + 1] != 0.f ? hyper[2] : 0.f;
-    const int scrub = (int)seg_table[4 * seg + 2];
-    const size_t i = ((size_t)blockIdx.x * TB + threadIdx.x) * 4;
+    int block = blockIdx.x;
+    for (int k = 0; k < done.ranges && block >= done.first[k]; ++k) block += done.count[k];
+    const int seg = block_seg[block];
+    const SgdStep s = sgd_step(seg_table + 4 * seg, hyper);
+    const size_t i = ((size_t)block * TB + threadIdx.x) * 4;
     float4 w = ld4(W + i), u = ld4(U + i), g = ld4(G + i);
-    const size_t b0 = (size_t)blockIdx.x * TB * 4;
+    const size_t b0 = (size_t)block * TB * 4;
     if (t.world > 1) {
         // A peer's gradients never arrived (tail_wait_kernel gave up): no block updates anything, so that the
         // parameters of this rank stay those of the last complete step.
@@ -1485,18 +1475,17 @@ __global__ void __launch_bounds__(TB) sgd_arena_kernel(float *W, float *U, float
         }
     }
     u.x += g.x; u.y += g.y; u.z += g.z; u.w += g.w;
-    if (frozen) {
+    if (s.frozen) {   // not updated now: the gradient joins the pending update, nothing else moves
         st4(U + i, u);
         st4(G + i, make_float4(0.f, 0.f, 0.f, 0.f));
         return;
     }
-    if (scrub) {
+    if (s.scrub) {
         const size_t first = (size_t)__float_as_int(seg_table[4 * seg + 3]) * TB * 4;
-        if (scrub4(w, u, scrub, i - first) && status) atomicOr(status, AET_STATUS_NAN);
+        if (scrub4(w, u, s.scrub, i - first) && status) atomicOr(status, AET_STATUS_NAN);
     }
-    u.x += decay_term * w.x; u.y += decay_term * w.y; u.z += decay_term * w.z; u.w += decay_term * w.w;
-    w.x += rate * u.x; w.y += rate * u.y; w.z += rate * u.z; w.w += rate * u.w;
-    u.x *= momentum; u.y *= momentum; u.z *= momentum; u.w *= momentum;
+    sgd_move(w.x, u.x, s.rate, s.momentum, s.decay); sgd_move(w.y, u.y, s.rate, s.momentum, s.decay);
+    sgd_move(w.z, u.z, s.rate, s.momentum, s.decay); sgd_move(w.w, u.w, s.rate, s.momentum, s.decay);
     st4(W + i, w);
     st4(U + i, u);
     st4(G + i, make_float4(0.f, 0.f, 0.f, 0.f));
@@ -1554,9 +1543,8 @@ __global__ void sgd_segment_kernel(float *W, float *U, float *G, size_t n4, floa
     float4 w = ld4(W + i), u = ld4(U + i), g = ld4(G + i);
     u.x += g.x; u.y += g.y; u.z += g.z; u.w += g.w;
     if (scrub && scrub4(w, u, scrub, i) && status) atomicOr(status, AET_STATUS_NAN);
-    u.x += decay_term * w.x; u.y += decay_term * w.y; u.z += decay_term * w.z; u.w += decay_term * w.w;
-    w.x += rate * u.x; w.y += rate * u.y; w.z += rate * u.z; w.w += rate * u.w;
-    u.x *= momentum; u.y *= momentum; u.z *= momentum; u.w *= momentum;
+    sgd_move(w.x, u.x, rate, momentum, decay_term); sgd_move(w.y, u.y, rate, momentum, decay_term);
+    sgd_move(w.z, u.z, rate, momentum, decay_term); sgd_move(w.w, u.w, rate, momentum, decay_term);
     st4(W + i, w);
     st4(U + i, u);
     st4(G + i, make_float4(0.f, 0.f, 0.f, 0.f));
@@ -2371,7 +2359,16 @@ int k_comm_stamp(aet_context *ctx, unsigned long long *dev4, int after) {
 
 int k_sgd_arena(aet_network *net) {
     aet_context *ctx = net->ctx;
-    LaunchScope s(ctx, "sgd_momentum", 24.0 * net->arena.used, 0);
+    UpdatedBlocks done = {};
+    int blocks = net->n_blocks;
+    for (aet_layer *l : net->layers) {   // in the arena's order
+        if (!l->updated) continue;
+        l->updated = false;
+        done.first[done.ranges] = (int)(l->seg_w.offset / 1024);
+        done.count[done.ranges] = (int)(l->seg_w.padded / 1024);
+        blocks -= done.count[done.ranges++];
+    }
+    LaunchScope s(ctx, "sgd_momentum", 24.0 * 1024.0 * blocks, 0);
     TailArgs t = {};
     if (net->xchg_active && net->tail_n) {
         for (int q = 0; q < net->world; ++q) t.peer_buf[q] = reinterpret_cast<const float *>(net->xchg_peer[q] + kXchgFlagBytes);
@@ -2386,8 +2383,8 @@ int k_sgd_arena(aet_network *net) {
         AET_TRY(aet_check_launch("grad_wait"));
     }
     net->comm_stamped = false;
-    launch_k(ctx->stream, net->n_blocks, TB, 0, sgd_arena_kernel, net->arena.W, net->arena.U, net->arena.G, net->block_seg,
-                                                           net->seg_table, net->hyper_dev, t, ctx->status_dev);
+    launch_k(ctx->stream, blocks, TB, 0, sgd_arena_kernel, net->arena.W, net->arena.U, net->arena.G, net->block_seg, net->seg_table,
+             net->hyper_dev, done, t, ctx->status_dev);
     return aet_check_launch("sgd_momentum");
 }
 

@@ -537,9 +537,19 @@ extern "C" int aet_layer_backward(aet_layer *l, aet_state state) {
             if (l->bn) AET_TRY(k_bn_backward(l, nullptr));
             else AET_TRY(k_bias_act_backward(l));
         }
+        const bool update = conv_update_ok(l);
+        if (update && pd) {   // the data gradient reads the weights that the weight gradient's epilogue is going to move
+            AET_TRY(conv_dgrad(l, l->delta->d, pd->d));
+            pd->lazy_zero = false;
+        }
         // In a network's backward pass the weight gradient runs on the side stream, beside the
         // data-gradient chain of this and the earlier layers (both only read this layer's delta).
         if (l->ctx->overlap_wgrad) AET_TRY(side_begin(l->ctx));
+        if (update) {
+            const int ur = conv_wgrad_update(l, state.input->d, l->delta->d);
+            side_end(l->ctx);
+            return ur;
+        }
         const int wr = conv_wgrad(l, state.input->d, l->delta->d, layer_G(l), l->ctx->wgrad_fresh ? 0 : 1);
         side_end(l->ctx);
         AET_TRY(wr);

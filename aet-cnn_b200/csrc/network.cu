@@ -185,6 +185,7 @@ int build_sgd_tables(aet_network *net) {
             if (!segs[k]) continue;
             if (segs[k]->offset != block_seg.size() * 1024) { aet_set_error("internal: arena segments are not contiguous"); return AET_E_INVALID; }
             const int first_block = (int)block_seg.size();
+            if (k == 0) l->seg_id = seg_id;
             for (size_t b = 0; b < segs[k]->padded / 1024; ++b) block_seg.push_back(seg_id);
             // {learning-rate multiplier, decay flag, non-finite scrub kind, first block of the segment (int bits)}
             const bool mtcs = net->ctx->parity == AET_PARITY_MTCS;
@@ -380,8 +381,13 @@ int run_step(aet_network *net, bool final) {
     st.input = net->input;
     // every update leaves the gradient arena zero, so without subdivisions this backward pass is the only writer of G
     net->ctx->wgrad_fresh = net->subdivisions == 1 && net->grad_clean;
+    // and where no other rank's gradients join in, nobody sees the gradient between this pass and the update
+    if (net->ctx->wgrad_fresh && final && !net->adam && !net->comm && !net->xchg_active) net->ctx->update_in = net;
     const int br = net_backward(net, st, final);
     net->ctx->wgrad_fresh = false;
+    net->ctx->update_in = nullptr;
+    if (br != AET_OK)
+        for (aet_layer *l : net->layers) l->updated = false;
     AET_TRY(br);
     net->grad_clean = false;
     if (!final) return AET_OK;   // gradients keep accumulating in the arena until the group's last call

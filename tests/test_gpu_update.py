@@ -1,0 +1,97 @@
+"""Training steps whose weight gradients apply the update in their epilogue, against the same step made call by call."""
+import os
+
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+from gpu_util import variants_used
+
+pytestmark = pytest.mark.gpu
+
+HEAD = "[net]\nbatch=%d\nwidth=%d\nheight=%d\nchannels=%d\nlearning_rate=0.05\nmomentum=0.9\ndecay=0.0005\npolicy=constant\n\n"
+CONV = "[convolutional]\nfilters=%d\nsize=%d\nstride=1\npad=%d\nactivation=%s\n%s\n"
+
+
+def two_nets(aet, ctx, text, batch):
+    rng = np.random.default_rng(batch)
+    nets = [aet.NNetwork(ctx, cfg_text=text, train=1, batch=batch) for _ in range(2)]
+    x = rng.random(nets[0].input_shape, np.float32)
+    t = np.eye(nets[0].outputs, dtype=np.float32)[rng.integers(0, nets[0].outputs, batch)]
+    for n in nets:
+        n.use_graph(False)
+        n.input.write(x)
+        n.truth.write(t)
+    return nets
+
+
+def step_by_calls(aet, net):
+    st = aet.make_state(input=net.input, truth=net.truth, train=1)
+    net.forward(st)
+    net.backward(aet.make_state(input=net.input, truth=net.truth, train=1))
+    net.update()
+
+
+def compare(aet, fused, plain, tol):
+    for i in range(fused.layer_count):
+        a, b = fused.layer(i), plain.layer(i)
+        for which in (aet.P_WEIGHTS, aet.P_WEIGHT_UPDATES, aet.P_BIASES, aet.P_BIAS_UPDATES):
+            if a.param_count(which):
+                u, v = a.read(which), b.read(which)
+                assert np.isfinite(u).all() and rel_l2(u, v) <= tol, (i, which, rel_l2(u, v))
+
+
+# (batch, map, channels, filters): one slab and eight of them, filters beside the tiles' widths, channels that end inside a block
+@pytest.mark.parametrize("shape", [(8, 8, 64, 257), (40, 7, 20, 1100), (128, 8, 64, 1000), (256, 6, 128, 400)])
+@pytest.mark.parametrize("graph", [False, True])
+def test_fully_connected_layers_update_themselves(aet, ctx, shape, graph):
+    """Same products in the same precision; the sums of a split gradient and of one that is not differ by rounding, a few
+    times 1e-7 of a gradient, which the second step's forward pass carries on."""
+    batch, side, channels, filters = shape
+    text = (HEAD % (batch, side, side, 32) + CONV % (channels, 3, 1, "leaky", "") + CONV % (filters, side, 0, "relu", "learning_rate=0.5\n") +
+            CONV % (10, 1, 0, "linear", "") + "[softmax]\n")
+    fused, plain = two_nets(aet, ctx, text, batch)
+    try:
+        ctx.profile(0 if graph else 1)
+        fused.use_graph(graph)
+        for _ in range(3):
+            fused.train_device()
+            step_by_calls(aet, plain)
+        if not graph:
+            assert any("_sgd" in n for n in variants_used(ctx)), variants_used(ctx)
+        compare(aet, fused, plain, 2e-5)
+    finally:
+        ctx.profile(0)
+        fused.close()
+        plain.close()
+
+
+def test_self_updating_layers_scrub_and_hold_still(aet, ctx):
+    """Non-finite pending updates are cleared as by the update kernel, and a layer that is not updated yet only collects."""
+    for extra in ("", "dont_update=1\n"):
+        text = HEAD % (16, 8, 8, 32) + CONV % (64, 3, 1, "leaky", "") + CONV % (300, 8, 0, "relu", extra) + CONV % (10, 1, 0, "linear", "") + "[softmax]\n"
+        fused, plain = two_nets(aet, ctx, text, 16)
+        try:
+            for n in (fused, plain):
+                u = n.layer(1).read(aet.P_WEIGHT_UPDATES)
+                u[[3, 1017, len(u) - 1]] = np.nan, np.inf, -np.inf
+                if not extra:
+                    n.layer(1).write(aet.P_WEIGHT_UPDATES, u)
+            start = fused.layer(1).read(aet.P_WEIGHTS)
+            for step in range(2):
+                fused.train_device()
+                if not extra and step == 0:
+                    with pytest.raises(aet.AetError):
+                        ctx.check()
+                if extra:   # iteration 1: held
+                    assert np.array_equal(fused.layer(1).read(aet.P_WEIGHTS), start) == (step == 0)
+                    continue
+                step_by_calls(aet, plain)
+                if step == 0:
+                    with pytest.raises(aet.AetError):
+                        ctx.check()
+            if not extra:
+                compare(aet, fused, plain, 2e-5)
+        finally:
+            fused.close()
+            plain.close()
