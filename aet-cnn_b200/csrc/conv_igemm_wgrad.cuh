@@ -33,34 +33,31 @@ struct IgemmWgradArgs {
     unsigned long long *span;
 };
 
-constexpr int IG_UPDATERS = 12;   // UPDATE: epilogue warps, three to a quarter of the lanes
+constexpr int IG_UPDATERS = 16;   // UPDATE: epilogue warps, four to a quarter of the lanes
 
-// 32 channels (the lanes) of 16 filters, `off` bytes into the segment and `ld` bytes from one filter to the next: all loads are
-// in flight before the first is used.  FULL: all 16 filters exist.
-template <bool FULL>
-__device__ __forceinline__ bool update_rows(float *W, float *U, uint32_t off, uint32_t ld, int rows, const uint32_t (&g)[16], const SgdStep &s) {
-    char *wb = reinterpret_cast<char *>(W), *ub = reinterpret_cast<char *>(U);
-    float w[16], u[16];
+// One weight: 32 channels are the lanes.
+__device__ __forceinline__ bool update_one(float *W, float *U, uint32_t at, float w, float u, uint32_t g, const SgdStep &s) {
     bool hit = false;
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-        if (!FULL && k >= rows) break;
-        w[k] = __ldcs(reinterpret_cast<const float *>(wb + (off + k * ld)));
-        u[k] = __ldcs(reinterpret_cast<const float *>(ub + (off + k * ld)));
+    u += __uint_as_float(g);
+    if (!s.frozen) {
+        // one addition tells whether both are finite (or large enough for a closer look)
+        if (s.scrub && !(fabsf(u) + fabsf(w) <= FLT_MAX)) hit = scrub1(w, u, s.scrub, at / 4);
+        sgd_move(w, u, s.rate, s.momentum, s.decay);
+        __stcs(reinterpret_cast<float *>(reinterpret_cast<char *>(W) + at), w);
     }
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-        if (!FULL && k >= rows) break;
-        u[k] += __uint_as_float(g[k]);
-        if (!s.frozen) {
-            // one addition tells whether both are finite (or large enough for a closer look)
-            if (s.scrub && !(fabsf(u[k]) + fabsf(w[k]) <= FLT_MAX)) hit |= scrub1(w[k], u[k], s.scrub, (off + k * ld) / 4);
-            sgd_move(w[k], u[k], s.rate, s.momentum, s.decay);
-            __stcs(reinterpret_cast<float *>(wb + (off + k * ld)), w[k]);
-        }
-        __stcs(reinterpret_cast<float *>(ub + (off + k * ld)), u[k]);
-    }
+    __stcs(reinterpret_cast<float *>(reinterpret_cast<char *>(U) + at), u);
     return hit;
+}
+// The weights and momenta of eight filters, `off` bytes into the segment and `ld` bytes from one filter to the next.
+struct UpdateRows {
+    float w[8], u[8];
+};
+__device__ __forceinline__ void update_load(UpdateRows &r, const float *W, const float *U, uint32_t off, uint32_t ld) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        r.w[k] = __ldcs(reinterpret_cast<const float *>(reinterpret_cast<const char *>(W) + (off + k * ld)));
+        r.u[k] = __ldcs(reinterpret_cast<const float *>(reinterpret_cast<const char *>(U) + (off + k * ld)));
+    }
 }
 
 template <bool PAIR, bool X3, bool UPDATE>
@@ -115,8 +112,8 @@ conv_wgrad_igemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
     const int step = X3 ? a.chunk_slabs : a.slabs_per_split;
 
     if (UPDATE && (warp < 4 || warp >= 8)) {
-        // ------------------------------------------------------------------ epilogue that updates the weights (warps 0-3, 8-15)
-        const int quarter = warp & 3, share = warp < 4 ? 0 : (warp - 4) >> 2;   // this warp's lanes, and which 16 of 48 filters
+        // ------------------------------------------------------------------ epilogue that updates the weights (warps 0-3, 8-19)
+        const int quarter = warp & 3, share = warp < 4 ? 0 : (warp - 4) >> 2;   // this warp's lanes, and which 8 of 32 filters
         const SgdStep s = sgd_step(a.seg, a.hyper);
         const uint32_t ld = (uint32_t)a.out_ld * 4u;
         bool hit = false;
@@ -126,22 +123,43 @@ conv_wgrad_igemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
             const int blk = mt * 4 + quarter, tap = blk / a.blocks_per_tap, c = (blk - tap * a.blocks_per_tap) * 32 + lane;
             const bool live = blk < a.blocks && c < a.cp;
             const int n0 = nt * a.bn;
+            // This warp's filters come in eights: the first are asked for in front of the wait for the products, each next eight
+            // before the current ones are used.
+            const int rows = live ? a.filters - n0 : 0;
+            const uint32_t off0 = (uint32_t)n0 * ld + (uint32_t)(tap * a.cp + c) * 4u;
+            UpdateRows r[2];
+            int c0 = share * 8;
+            if (c0 + 8 <= rows && c0 < a.bn) update_load(r[0], a.W, a.U, off0 + (uint32_t)c0 * ld, ld);
             const uint32_t b = tcount & 1u;
             bool ok = mbar_wait(smem_u32(&ctl.acc_full[b]), (tcount >> 1) & 1u, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after_sync();
             const uint32_t src = tmem + b * (uint32_t)a.bn + ((uint32_t)(quarter * 32) << 16);
-            for (int c0 = share * 16; c0 < a.bn; c0 += IG_UPDATERS * 4) {
+            auto turn = [&](UpdateRows &now, UpdateRows &next) {
+                const int c1 = c0 + IG_UPDATERS / 4 * 8;
+                if (c1 + 8 <= rows && c1 < a.bn) update_load(next, a.W, a.U, off0 + (uint32_t)c1 * ld, ld);
+                uint32_t v[8];
                 __syncwarp();
-                uint32_t v[16];
-                tmem_ld16_issue(src + (uint32_t)c0, v);
-                tmem_ld_wait();
-                const int rows = a.filters - n0 - c0;
-                const uint32_t off = (uint32_t)(n0 + c0) * ld + (uint32_t)(tap * a.cp + c) * 4u;
-                if (!live || rows <= 0) continue;
-                if (rows >= 16) hit |= update_rows<true>(a.W, a.U, off, ld, 16, v, s);
-                else hit |= update_rows<false>(a.W, a.U, off, ld, rows, v, s);
+                tmem_ld8(src + (uint32_t)c0, v);
+                const uint32_t off = off0 + (uint32_t)c0 * ld;
+                if (c0 + 8 <= rows) {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) hit |= update_one(a.W, a.U, off + k * ld, now.w[k], now.u[k], v[k], s);
+                } else {   // the last filters, fewer than eight
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        if (c0 + k < rows) {
+                            const uint32_t at = off + k * ld;
+                            hit |= update_one(a.W, a.U, at, *reinterpret_cast<const float *>(reinterpret_cast<const char *>(a.W) + at),
+                                              *reinterpret_cast<const float *>(reinterpret_cast<const char *>(a.U) + at), v[k], s);
+                        }
+                }
+                c0 = c1;
+            };
+            while (c0 < a.bn) {
+                turn(r[0], r[1]);
+                if (c0 < a.bn) turn(r[1], r[0]);
             }
             tc_fence_before_sync();
             __syncwarp();
@@ -463,7 +481,8 @@ int igemm_wgrad(aet_layer *l, const ConvArgs &ca, float *dw, int accumulate, dou
 // Fully connected layers in a training step: the weight gradient's epilogue applies the update.  A gradient as large as the
 // weights, from a batch that is a few K slabs, is bound by memory: written, read again and cleared by the update it costs
 // 28 bytes per weight (4096 x 9216 at batch 128: 100 us alone and 157 of the update's 255), in the epilogue the 16 that the
-// weights and their momentum take (164 us; a step of the 227x227 network 2.31 -> 2.17 ms).  From a million weights on and up to
+// weights and their momentum take (16 warps with eight rows each in flight 124 us, 5.3 TB/s; 12 warps with sixteen rows asked
+// for after the products 164; eight steps of the 227x227 network 18.33 -> 17.55 -> 17.22 ms).  From a million weights on and up to
 // 8 slabs (256 images); below that, or where K is longer, the launch and the products count.  Offsets are 32 bits of bytes.
 bool igemm_update_ok(const aet_layer *l, const ConvGeom &g) {
     Im2colBox box;
