@@ -127,6 +127,7 @@ struct aet_context {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_gram = nullptr;   // ev_gram: the Gram matrix of this pass's input patches is there
     bool overlap_wgrad = false;   // set by the network around its backward pass
     bool wgrad_fresh = false;     // set by a training step without subdivisions: the gradient arena is zero when backward starts, the weight gradients may overwrite
+    bool step_forward = false;          // a training step's forward pass, whose backward pass is queued right behind it
     aet_network *update_in = nullptr;   // set by a training step whose update follows at once: weight gradients may apply it themselves
     bool on_side = false, side_pending = false;
     float *scratch_side = nullptr;
@@ -240,6 +241,7 @@ struct aet_layer {
     bool lin_head = false;           // eligible (set when the network is wired)
     bool lin_fwd_pending = false;    // forward deferred to the softmax layer's call
     bool lin_used = false;           // the last forward went through the fused kernel
+    bool lin_dx_done = false;        // ... and has formed the delta of this layer's input, for the backward pass of the same step
     bool lin_out_stale = false;      // output tensor not formed (a host tap runs the convolution)
     bool lin_bwd_pending = false;    // softmax/avg-pool backward deferred to this layer's backward call
     bool lin_delta_stale = false;    // delta tensor not formed (a host tap broadcasts it)
@@ -575,7 +577,7 @@ int k_avgpool_backward(aet_layer *l, float *prev_delta, int accumulate);
 int k_softmax_forward(aet_layer *l, const float *x, const float *truth);
 int k_head_forward(aet_layer *conv, aet_layer *avg, aet_layer *sm, const float *truth);
 int k_head_backward(aet_layer *conv, aet_layer *avg, aet_layer *sm);
-int k_linhead_forward(aet_layer *conv, aet_layer *avg, aet_layer *sm, const float *x, const float *truth);
+int k_linhead_forward(aet_layer *conv, aet_layer *avg, aet_layer *sm, const float *x, const float *truth, float *pd);
 int k_linhead_backward(aet_layer *conv, aet_layer *avg, aet_layer *sm, float *pd);
 int k_linhead_conv_delta(aet_layer *conv, aet_layer *avg, aet_layer *sm);
 int k_axpy(aet_context *ctx, float *y, const float *x, float a, size_t n, int accumulate, const char *name);

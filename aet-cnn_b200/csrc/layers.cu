@@ -401,7 +401,7 @@ extern "C" int aet_layer_forward(aet_layer *l, aet_state state) {
                 l->output_stale = false;
             }
         } else {
-            l->lin_used = false; l->lin_out_stale = false; l->lin_delta_stale = false; l->lin_bwd_pending = false;
+            l->lin_used = false; l->lin_out_stale = false; l->lin_delta_stale = false; l->lin_bwd_pending = false; l->lin_dx_done = false;
             if (l->lin_head && l->ctx->in_network_pass && (state.train ? state.truth != nullptr : l->index > 0)) {
                 // classifier head of a network: folded into the softmax layer's call.  (A prediction's output has to stay
                 // what it was until somebody reads it: where the input is the caller's tensor, nothing here sees that change.)
@@ -445,7 +445,9 @@ extern "C" int aet_layer_forward(aet_layer *l, aet_state state) {
             cv->lin_fwd_pending = false;
             if (l->head_avg->head_forward_pending && state.input == l->head_avg->output) {
                 l->head_avg->head_forward_pending = false;
-                AET_TRY(k_linhead_forward(cv, l->head_avg, l, cv->lin_input->d, truth));
+                aet_tensor *pd = truth && l->ctx->step_forward && l->net && cv->index > 0 ? l->net->layers[cv->index - 1]->delta : nullptr;
+                AET_TRY(k_linhead_forward(cv, l->head_avg, l, cv->lin_input->d, truth, pd ? pd->d : nullptr));
+                cv->lin_dx_done = pd != nullptr;
                 cv->lin_used = truth != nullptr;
                 cv->lin_out_stale = true;
                 if (truth) l->delta->lazy_zero = false;
@@ -495,7 +497,13 @@ extern "C" int aet_layer_backward(aet_layer *l, aet_state state) {
             // fused linear head: softmax and avg-pool backward, this layer's data, weight and bias gradients in one kernel
             l->lin_bwd_pending = false;
             if (!pd) return fail_invalid("linear head backward needs the previous layer's delta");
-            AET_TRY(k_linhead_backward(l, l->head_softmax->head_avg, l->head_softmax, pd->d));
+            // what is left of a delta that came with the forward pass is for the update alone
+            const bool ahead = l->lin_dx_done;
+            l->lin_dx_done = false;
+            if (ahead && l->ctx->overlap_wgrad) AET_TRY(side_begin(l->ctx));
+            const int hr = k_linhead_backward(l, l->head_softmax->head_avg, l->head_softmax, ahead ? nullptr : pd->d);
+            side_end(l->ctx);
+            AET_TRY(hr);
             pd->lazy_zero = false;
             l->delta->lazy_zero = false;
             l->lin_delta_stale = true;

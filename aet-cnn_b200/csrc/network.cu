@@ -377,7 +377,10 @@ int net_backward(aet_network *net, aet_state state, bool exchange = true) {
 int run_step(aet_network *net, bool final) {
     aet_state st = {};
     st.truth = net->truth; st.input = net->input; st.delta = nullptr; st.train = 1;
-    AET_TRY(net_forward(net, st));
+    net->ctx->step_forward = true;
+    const int fr = net_forward(net, st);
+    net->ctx->step_forward = false;
+    AET_TRY(fr);
     st.input = net->input;
     // every update leaves the gradient arena zero, so without subdivisions this backward pass is the only writer of G
     net->ctx->wgrad_fresh = net->subdivisions == 1 && net->grad_clean;

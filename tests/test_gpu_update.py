@@ -95,3 +95,47 @@ def test_self_updating_layers_scrub_and_hold_still(aet, ctx):
         finally:
             fused.close()
             plain.close()
+
+
+IMAGE_NET = ("[net]\nbatch=%d\nwidth=%d\nheight=%d\nchannels=%d\nparity=%s\nlearning_rate=0.01\nmomentum=0.9\ndecay=0.0005\npolicy=constant\n\n"
+             "[convolutional]\nfilters=%d\nsize=3\nstride=1\npad=1\nbatch_normalize=1\nactivation=leaky\n\n[maxpool]\nsize=2\nstride=2\n\n"
+             "[convolutional]\nfilters=%d\nsize=3\nstride=1\npad=1\nbatch_normalize=1\nactivation=leaky\n\n[maxpool]\nsize=2\nstride=2\n\n"
+             "[convolutional]\nfilters=%d\nsize=1\nstride=1\npad=0\nactivation=linear\n\n[avgpool]\n\n[softmax]\ngroups=1\n")
+
+
+def compare_all(aet, fused, plain, tol):
+    for i in range(fused.layer_count):
+        a, b = fused.layer(i), plain.layer(i)
+        for which in (aet.P_WEIGHTS, aet.P_WEIGHT_UPDATES, aet.P_BIASES, aet.P_BIAS_UPDATES, aet.P_SCALES, aet.P_SCALE_UPDATES, aet.P_ROLLING_MEAN,
+                      aet.P_DELTA, aet.P_OUTPUT):
+            if a.param_count(which):
+                u, v = a.read(which), b.read(which)
+                assert np.isfinite(u).all() and rel_l2(u, v) <= tol, (i, which, rel_l2(u, v))
+
+
+# (batch, map, image channels, filters of the first and second layer, classes, parity)
+@pytest.mark.parametrize("case", [(37, 32, 3, 64, 128, 10, "mtcs"), (5, 24, 1, 128, 96, 3, "cpu"), (9, 36, 2, 61, 260, 32, "mtcs")])
+@pytest.mark.parametrize("graph", [False, True])
+def test_head_delta_with_the_forward_pass(aet, ctx, case, graph):
+    """In a training step the classifier head forms its input's delta with the forward pass.  The same numbers are added up in
+    the same order as call by call; what the compiler contracts differently in the two forms is a rounding of a delta."""
+    batch, side, channels, n0, n1, classes, parity = case
+    text = IMAGE_NET % (batch, side, side, channels, parity, n0, n1, classes)
+    fused, plain = two_nets(aet, ctx, text, batch)
+    try:
+        fused.use_graph(graph)
+        ctx.profile(0 if graph else 1)
+        for _ in range(2):
+            fused.train_device()
+            step_by_calls(aet, plain)
+        if not graph:
+            names = variants_used(ctx)
+            assert any(n.startswith("linear_head_forward.dx") for n in names), names
+        # of values that differ in the last of 24 bits one in 2^13 falls on the other side of a TF32 step of 2^-10 of its size:
+        # sqrt(2^-13) 2^-10 = 1.1e-5 for each of the three convolutions that such a value passes
+        compare_all(aet, fused, plain, 3.3e-5)
+    finally:
+        ctx.profile(0)
+        ctx.set_parity(aet.PARITY_MTCS)
+        fused.close()
+        plain.close()
