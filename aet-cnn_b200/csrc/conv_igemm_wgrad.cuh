@@ -60,8 +60,14 @@ __device__ __forceinline__ void update_load(UpdateRows &r, const float *W, const
     }
 }
 
+template <bool X3, bool UPDATE>
+struct IgemmWgradWarps {
+    static constexpr int groups = X3 || UPDATE ? 1 : 2;   // of four epilogue warps: the second is warps 8-11
+    static constexpr int threads = 256 + (X3 ? IG_CONVERTERS * 32 : (UPDATE ? (IG_UPDATERS - 4) * 32 : 128));
+};
+
 template <bool PAIR, bool X3, bool UPDATE>
-__global__ void __launch_bounds__(256 + (X3 ? IG_CONVERTERS * 32 : (UPDATE ? (IG_UPDATERS - 4) * 32 : 0)), 1)
+__global__ void __launch_bounds__(IgemmWgradWarps<X3, UPDATE>::threads, 1)
 conv_wgrad_igemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_dy, const IgemmWgradArgs a) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ IgemmCtl ctl;
@@ -83,7 +89,7 @@ conv_wgrad_igemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&ctl.acc_full[b]), 1);
-            mbar_init(smem_u32(&ctl.acc_empty[b]), UPDATE ? IG_UPDATERS : (PAIR ? 8 : 4));
+            mbar_init(smem_u32(&ctl.acc_empty[b]), UPDATE ? IG_UPDATERS : (PAIR ? 8 : 4) * IgemmWgradWarps<X3, UPDATE>::groups);
         }
         ctl.abort_flag = 0;
         fence_barrier_init();
@@ -166,13 +172,17 @@ conv_wgrad_igemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
             if (lane == 0) mbar_arrive(smem_u32(&ctl.acc_empty[b]));
         }
         if (hit && a.status) atomicOr(a.status, AET_STATUS_NAN);
-    } else if (warp < 4) {
+    } else if (warp < 4 || (IgemmWgradWarps<X3, UPDATE>::groups == 2 && warp >= 8)) {
         // ------------------------------------------------------------------ epilogue: a warp's 32 lanes are one 32-channel block
+        // Two groups of warps take every other 32 filters: the instructions of a lone warp per scheduler take 3.6 us for a tile of
+        // 64 filters, more than the products of a small layer (64 -> 64 on 24x24, batch 32: 13.9 -> 12.0 us).
+        constexpr int GROUPS = IgemmWgradWarps<X3, UPDATE>::groups;
+        const int quarter = warp & 3, group = warp < 4 ? 0 : 1;
         uint32_t tcount = 0;
         bool ok = true;
         for (int t = unit; t < total_tiles && ok; t += units) {
             const int sp = split_of(t), q = t - sp * per_split, nt = q / a.m_tiles, mt = q - nt * a.m_tiles;
-            const int blk = mt * (PAIR ? 8 : 4) + (int)prank * 4 + warp;
+            const int blk = mt * (PAIR ? 8 : 4) + (int)prank * 4 + quarter;
             const int tap = blk / a.blocks_per_tap, c = (blk - tap * a.blocks_per_tap) * 32 + lane;
             const bool live = blk < a.blocks && c < a.cp;
             const int n0 = nt * a.bn;
@@ -185,8 +195,8 @@ conv_wgrad_igemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc_fence_after_sync();
-                const uint32_t src = tmem + b * (uint32_t)a.bn + ((uint32_t)(warp * 32) << 16);
-                for (int c0 = 0; c0 < a.bn; c0 += 32) {
+                const uint32_t src = tmem + b * (uint32_t)a.bn + ((uint32_t)(quarter * 32) << 16);
+                for (int c0 = group * 32; c0 < a.bn; c0 += 32 * GROUPS) {
                     uint32_t v[32];
                     if (have) {
                         tmem_ld16_issue(src + (uint32_t)c0, v);
@@ -200,11 +210,25 @@ conv_wgrad_igemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
 #pragma unroll
                         for (int k = 0; k < 32; ++k)
                             if (live && n0 + c0 + k < a.filters) atomicAdd(dst + (size_t)(c0 + k) * a.out_ld, __uint_as_float(v[k]));
-                    } else if (live) {
+                    } else if (X3) {
+                        if (live) {
 #pragma unroll
-                        for (int k = 0; k < 32; ++k)
-                            if (n0 + c0 + k < a.filters) dst[(size_t)(c0 + k) * a.out_ld] = __uint_as_float(v[k]);
+                            for (int k = 0; k < 32; ++k)
+                                if (n0 + c0 + k < a.filters) dst[(size_t)(c0 + k) * a.out_ld] = __uint_as_float(v[k]);
+                        }
+                    } else if (live) {
+                        float *at = dst + (size_t)c0 * a.out_ld;
+                        const int rows = a.filters - n0 - c0;
+                        if (rows >= 32) {
+#pragma unroll
+                            for (int k = 0; k < 32; ++k, at += a.out_ld) *at = __uint_as_float(v[k]);
+                        } else {
+#pragma unroll
+                            for (int k = 0; k < 32; ++k, at += a.out_ld)
+                                if (k < rows) *at = __uint_as_float(v[k]);
+                        }
                     }
+                    if (!X3) __syncwarp();   // the next loads from the accumulator are the whole warp's
                 }
                 tc_fence_before_sync();
                 __syncwarp();
@@ -265,7 +289,7 @@ conv_wgrad_igemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
                 }
             }
         }
-    } else if (warp < 8) {
+    } else if (warp >= 5 && warp < 8) {
         // ------------------------------------------------------------------ copies: two activation blocks each (warps 5, 6), delta (warp 7)
         if (lane == 0) {
             const uint32_t full0 = smem_u32(&ctl.full[0]), empty0 = smem_u32(&ctl.empty[0]);
@@ -401,8 +425,8 @@ int igemm_wgrad_launch(aet_context *ctx, const CUtensorMap &mx, const CUtensorMa
     const int grid = (tiles < units ? tiles : units) * (PAIR ? 2 : 1);
     LaunchScope scope(ctx, "conv_wgrad_tma", 0, flops, variant);
     a.span = ctx->span_ptr;
-    if (PAIR) launch_k_cluster(ctx->stream, dim3(grid), dim3(256 + (X3 ? IG_CONVERTERS * 32 : (UPDATE ? (IG_UPDATERS - 4) * 32 : 0))), smem_bytes, 2, 1, conv_wgrad_igemm_kernel<PAIR, X3, UPDATE>, mx, mdy, a);
-    else launch_k(ctx->stream, dim3(grid), dim3(256 + (X3 ? IG_CONVERTERS * 32 : (UPDATE ? (IG_UPDATERS - 4) * 32 : 0))), smem_bytes, conv_wgrad_igemm_kernel<PAIR, X3, UPDATE>, mx, mdy, a);
+    if (PAIR) launch_k_cluster(ctx->stream, dim3(grid), dim3(IgemmWgradWarps<X3, UPDATE>::threads), smem_bytes, 2, 1, conv_wgrad_igemm_kernel<PAIR, X3, UPDATE>, mx, mdy, a);
+    else launch_k(ctx->stream, dim3(grid), dim3(IgemmWgradWarps<X3, UPDATE>::threads), smem_bytes, conv_wgrad_igemm_kernel<PAIR, X3, UPDATE>, mx, mdy, a);
     return aet_check_launch("conv_wgrad_tma");
 }
 
