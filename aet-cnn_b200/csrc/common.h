@@ -128,6 +128,7 @@ struct aet_context {
     bool overlap_wgrad = false;   // set by the network around its backward pass
     bool wgrad_fresh = false;     // set by a training step without subdivisions: the gradient arena is zero when backward starts, the weight gradients may overwrite
     bool step_forward = false;          // a training step's forward pass, whose backward pass is queued right behind it
+    bool in_step = false;               // a training step's backward pass, right behind its forward pass
     aet_network *update_in = nullptr;   // set by a training step whose update follows at once: weight gradients may apply it themselves
     bool on_side = false, side_pending = false;
     float *scratch_side = nullptr;

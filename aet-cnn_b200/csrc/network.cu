@@ -386,7 +386,9 @@ int run_step(aet_network *net, bool final) {
     net->ctx->wgrad_fresh = net->subdivisions == 1 && net->grad_clean;
     // and where no other rank's gradients join in, nobody sees the gradient between this pass and the update
     if (net->ctx->wgrad_fresh && final && !net->adam && !net->comm && !net->xchg_active) net->ctx->update_in = net;
+    net->ctx->in_step = true;
     const int br = net_backward(net, st, final);
+    net->ctx->in_step = false;
     net->ctx->wgrad_fresh = false;
     net->ctx->update_in = nullptr;
     if (br != AET_OK)

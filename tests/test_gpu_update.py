@@ -139,3 +139,34 @@ def test_head_delta_with_the_forward_pass(aet, ctx, case, graph):
         ctx.set_parity(aet.PARITY_MTCS)
         fused.close()
         plain.close()
+
+
+@pytest.mark.parametrize("case", [(3, 3, 2, "leaky", 0, 27, 96), (2, 2, 2, "relu", 0, 16, 20), (3, 3, 2, "linear", 0, 14, 33), (2, 2, 2, "leaky", 1, 15, 32),
+                                  (3, 3, 2, "tanh", 0, 13, 32)])
+@pytest.mark.parametrize("dropout", [False, True])
+def test_pool_backward_from_the_pooled_values(aet, ctx, case, dropout):
+    """The convolution in front of a max-pool (no batch norm) takes its activation's gradient from the pooled output in a training
+    step; not behind a dropout layer, which changes that output, and not for activations other than the simple ones."""
+    batch, size, stride, act, padding, side, filters = case
+    text = (HEAD % (batch + 2, side, side, 3) + CONV % (filters, 3, 1, act, "") + "[maxpool]\nsize=%d\nstride=%d\npadding=%d\n\n" % (size, stride, padding) +
+            ("[dropout]\nprobability=0.5\n\n" if dropout else "") + CONV % (10, 1, 0, "linear", "") + "[avgpool]\n\n[softmax]\n")
+    fused, plain = two_nets(aet, ctx, text, batch + 2)
+    try:
+        if dropout:
+            r = np.random.default_rng(7).random(fused.layer(2).param_count(aet.P_RAND), np.float32)
+            for n in (fused, plain):
+                n.layer(2).write(aet.P_RAND, r)
+        ctx.profile(1)
+        fused.train_device()
+        names = variants_used(ctx)
+        ctx.profile(0)
+        pooled = act != "tanh" and not dropout and padding // 2 == 0
+        assert any(n.startswith("pool_bias_act_bwd.pooled") for n in names) == pooled, names
+        step_by_calls(aet, plain)
+        compare(aet, fused, plain, 1e-6)
+        # up to four windows' deltas meet in a value, call by call in another order
+        assert rel_l2(fused.layer(0).read(aet.P_DELTA), plain.layer(0).read(aet.P_DELTA)) <= 4 * 2.0 ** -24
+    finally:
+        ctx.profile(0)
+        fused.close()
+        plain.close()
