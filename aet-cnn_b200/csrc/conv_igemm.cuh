@@ -10,6 +10,10 @@
 // What bounds it is the L2 -> SM path (52 to 60 bytes per clock and SM with all of them pulling), then the tensor pipe: a
 // 128 x 128 x 32 slab of TF32 brings 32 KB for 308 clocks of MMA.  So tiles are as large as the problem fills the chip with: a CTA pair
 // (cta_group::2) computes 256 pixels x up to 256 filters, each CTA fetching its own 128 pixels and half of the filters.
+// Where there are 128 columns or less, a CTA by itself does better with two M tiles (MT = 2) for one set of filters: 96 filters
+// bring 22 KB a tile and slab instead of 28, which a pair's 22 KB do not match (pairs get 47 bytes per clock where lone CTAs, whose
+// equal filters meet on the way, get 60).  5x5 taps, 256 -> 96 channels on 27x27, batch 128: 258 -> 230 us (as pairs 277); 3x3,
+// 48 -> 96 on 57x57: 125 -> 117; 96 filters at batch 50: 52 -> 46.
 // CTAs are persistent and hold two accumulators in TMEM: the epilogue of a tile (four warps) runs under the main loop
 // of the next.  The tiles of an incomplete last round are split along K over the chip and summed by the last to finish.
 //
@@ -124,9 +128,12 @@ __device__ __forceinline__ void igemm_low_halves(float4 *hi, uint32_t cells, uin
     }
 }
 
-template <int KIND, bool PAIR, bool X3>
+// MT: M tiles of 128 rows that a CTA computes side by side (2: not with pairs, not in 3xTF32, up to 128 columns)
+template <int KIND, bool PAIR, bool X3, int MT>
 __global__ void __launch_bounds__(224 + (X3 ? IG_CONVERTERS * 32 : 0), 1)
 conv_igemm_kernel(const __grid_constant__ IgemmMaps maps, const IgemmArgs a) {
+    static_assert(MT == 1 || (!PAIR && !X3), "two M tiles: single CTAs, TF32");
+    constexpr int ROWS = BM * (PAIR ? 2 : MT);   // of a tile
     constexpr int CHUNK = X3 ? 32 : IG_CHUNK, PITCH = CHUNK + 4;   // 3xTF32: the space is for a third stage
     extern __shared__ unsigned char smem_raw[];
     __shared__ IgemmCtl ctl;
@@ -137,12 +144,12 @@ conv_igemm_kernel(const __grid_constant__ IgemmMaps maps, const IgemmArgs a) {
     const bool leader = prank == 0u;
     const int units = (int)gridDim.x / (PAIR ? 2 : 1), unit = (int)blockIdx.x / (PAIR ? 2 : 1);
     const int total_tiles = a.direct_tiles + (a.m_tiles * a.n_tiles - a.direct_tiles) * a.parts;
-    constexpr uint32_t a_bytes = BM * BK * 4;
+    constexpr uint32_t a_bytes = MT * BM * BK * 4;
     const uint32_t half_bytes = a_bytes + a.b_bytes;               // both operands of a stage (this CTA's share)
     // A stage is two 32-deep slabs (one turn of a copying thread's loop costs it 260 clocks and more, the MMAs of a slab of
-    // 96 columns 300); 3xTF32: one slab, with the low halves of both operands behind it.
-    constexpr int KS = X3 ? 1 : 2;
-    const uint32_t stage_bytes = half_bytes * 2;
+    // 96 columns 300); 3xTF32: one slab, with the low halves of both operands behind it; two M tiles: one slab.
+    constexpr int KS = X3 || MT > 1 ? 1 : 2;
+    const uint32_t stage_bytes = half_bytes * (MT > 1 ? 1 : 2);
     float *staging = reinterpret_cast<float *>(smem_raw + (smem_base - smem_u32(smem_raw)) + (size_t)a.stages * stage_bytes);
 
     if (threadIdx.x == 0) {
@@ -175,11 +182,10 @@ conv_igemm_kernel(const __grid_constant__ IgemmMaps maps, const IgemmArgs a) {
     if (warp < 4) {
         // ------------------------------------------------------------------ epilogue
         float *mine = staging + (size_t)(warp * 32) * PITCH;
-        const size_t rows32 = (size_t)prank * 4 + warp;
         // Lane 0: this warp's place among the parts of its rows, the last one clears the ticket for the next launch.  A warp
         // whose wait ran out takes its tickets all the same: a part that did not would leave the next launch miscounting.
-        auto take_ticket = [&](int split) {
-            unsigned int *ticket = a.tickets + (size_t)split * (PAIR ? 8 : 4) + rows32;
+        auto take_ticket = [&](int split, int rows32) {
+            unsigned int *ticket = a.tickets + (size_t)split * (ROWS / 32) + rows32;
             const unsigned int order = atomicAdd(ticket, 1u);
             if (order == (unsigned)a.parts - 1u) *ticket = 0u;
             return order;
@@ -189,14 +195,6 @@ conv_igemm_kernel(const __grid_constant__ IgemmMaps maps, const IgemmArgs a) {
         for (int t = unit; t < total_tiles; t += units, ++tcount) {
             const IgemmTile tile = igemm_tile(a, t);
             const IgemmClass &cl = a.cls[tile.cls];
-            // this lane's row of the tile, and the output pixel it belongs to (-1: past the end)
-            const int row = tile.mt * (PAIR ? 256 : 128) + (int)prank * 128 + warp * 32 + lane;
-            int pix = row < cl.rows ? row : -1;
-            if (KIND == KIND_DGRAD && a.scatter > 1 && pix >= 0) {
-                const uint32_t n = fast_div((uint32_t)row, cl.div_hw), rem = (uint32_t)row - n * (uint32_t)cl.hw;
-                const uint32_t i = fast_div(rem, cl.div_w), j = rem - i * (uint32_t)cl.w;
-                pix = ((int)n * a.H + a.scatter * (int)i + cl.ph) * a.W + a.scatter * (int)j + cl.pw;
-            }
             if (KIND == KIND_FPROP) {   // the columns' constants come to L1 while the MMAs run
                 const int col = tile.n0 + lane * 32;
                 if (lane * 32 < a.bn && col < a.n_cols) {
@@ -208,150 +206,163 @@ conv_igemm_kernel(const __grid_constant__ IgemmMaps maps, const IgemmArgs a) {
             ok = ok && mbar_wait(smem_u32(&ctl.acc_full[b]), (tcount >> 1) & 1u, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) {
-                if (tile.split >= 0 && lane == 0) take_ticket(tile.split);
+                if (tile.split >= 0 && lane == 0)
+                    for (int h = 0; h < MT; ++h) take_ticket(tile.split, (PAIR ? (int)prank : h) * 4 + warp);
                 continue;
             }
             tc_fence_after_sync();
             const bool have = tile.slabs > 0;
-            const uint32_t acc = tmem + b * (uint32_t)a.bn + ((uint32_t)(warp * 32) << 16);
             const bool split = tile.split >= 0;
-            const float *parts = nullptr;              // this warp's rows of part 0: [column][lane]
-            const size_t part_stride = (size_t)a.bn * BM * (PAIR ? 2 : 1);
-            if (split) {
-                float *base = a.partial + (size_t)tile.split * a.parts * part_stride + rows32 * 32 * a.bn + lane;
-                float *mine_part = base + (size_t)tile.part * part_stride;
-                for (int c = 0; c < a.bn; c += 16) {
-                    uint32_t v[16];
-                    if (have) {
-                        tmem_ld16_issue(acc + (uint32_t)c, v);
-                        tmem_ld_wait();
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < 16; ++q) v[q] = 0u;
-                    }
-#pragma unroll
-                    for (int q = 0; q < 16; ++q) mine_part[(c + q) * 32] = __uint_as_float(v[q]);
+            const size_t part_stride = (size_t)a.bn * ROWS;
+#pragma unroll 1
+            for (int h = 0; h < MT; ++h) {
+                const int rows32 = (PAIR ? (int)prank : h) * 4 + warp;
+                // this lane's row of the tile, and the output pixel it belongs to (-1: past the end)
+                const int row = tile.mt * ROWS + rows32 * 32 + lane;
+                int pix = row < cl.rows ? row : -1;
+                if (KIND == KIND_DGRAD && a.scatter > 1 && pix >= 0) {
+                    const uint32_t n = fast_div((uint32_t)row, cl.div_hw), rem = (uint32_t)row - n * (uint32_t)cl.hw;
+                    const uint32_t i = fast_div(rem, cl.div_w), j = rem - i * (uint32_t)cl.w;
+                    pix = ((int)n * a.H + a.scatter * (int)i + cl.ph) * a.W + a.scatter * (int)j + cl.pw;
                 }
-                tc_fence_before_sync();
-                __threadfence();
-                __syncwarp();
-                unsigned int order = 0;
-                if (lane == 0) {
-                    if (PAIR) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl.acc_empty[b]), 0));
-                    else mbar_arrive(smem_u32(&ctl.acc_empty[b]));
-                    order = take_ticket(tile.split);
-                }
-                order = __shfl_sync(0xffffffffu, order, 0);
-                if (order != (unsigned)a.parts - 1u) continue;           // another part of these rows is still to come
-                __threadfence();
-                parts = base;
-            }
-            for (int c0 = 0; c0 < a.bn; c0 += CHUNK) {
-                const int w = a.bn - c0 < CHUNK ? a.bn - c0 : CHUNK;
+                const uint32_t acc = tmem + (b * MT + (uint32_t)h) * (uint32_t)a.bn + ((uint32_t)(warp * 32) << 16);
+                const float *parts = nullptr;              // this warp's rows of part 0: [column][lane]
+                if (split) {
+                    float *base = a.partial + (size_t)tile.split * a.parts * part_stride + rows32 * 32 * a.bn + lane;
+                    float *mine_part = base + (size_t)tile.part * part_stride;
+                    for (int c = 0; c < a.bn; c += 16) {
+                        uint32_t v[16];
+                        if (have) {
+                            tmem_ld16_issue(acc + (uint32_t)c, v);
+                            tmem_ld_wait();
+                        } else {
 #pragma unroll
-                for (int h = 0; h < CHUNK; h += 32) {
-                    if (h >= w) break;
-                    const bool second = h + 16 < w;
-                    uint32_t v[32];
-                    if (split) {
-                        float f[32];
-#pragma unroll
-                        for (int q = 0; q < 32; ++q) f[q] = 0.f;
-                        // several parts' loads in flight: a trip takes a round to L2
-                        constexpr int FLY = X3 ? 2 : 4;
-                        for (int p = 0; p < a.parts; p += FLY) {
-                            float g[FLY][32];
-#pragma unroll
-                            for (int u = 0; u < FLY; ++u) {
-                                const float *src = parts + (size_t)(p + u) * part_stride + (size_t)(c0 + h) * 32;
-#pragma unroll
-                                for (int q = 0; q < 32; ++q)
-                                    g[u][q] = (p + u < a.parts && (q < 16 || second)) ? __ldcg(src + q * 32) : 0.f;
-                            }
-#pragma unroll
-                            for (int u = 0; u < FLY; ++u)
-#pragma unroll
-                                for (int q = 0; q < 32; ++q) f[q] += g[u][q];
+                            for (int q = 0; q < 16; ++q) v[q] = 0u;
                         }
 #pragma unroll
-                        for (int q = 0; q < 32; ++q) v[q] = __float_as_uint(f[q]);
-                    } else if (have) {
-                        const uint32_t src = acc + (uint32_t)(c0 + h);
-                        tmem_ld16_issue(src, v);
-                        if (second) tmem_ld16_issue(src + 16u, v + 16);
-                        tmem_ld_wait();
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < 32; ++q) v[q] = 0u;
+                        for (int q = 0; q < 16; ++q) mine_part[(c + q) * 32] = __uint_as_float(v[q]);
                     }
-#pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        if (q < 4 || second)
-                            *reinterpret_cast<uint4 *>(mine + lane * PITCH + h + q * 4) = make_uint4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
-                }
-                if (!split && c0 + CHUNK >= a.bn) {   // the accumulator is read: the MMAs of the tile after the next may overwrite it
                     tc_fence_before_sync();
+                    __threadfence();
                     __syncwarp();
+                    unsigned int order = 0;
                     if (lane == 0) {
                         if (PAIR) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl.acc_empty[b]), 0));
-                        else mbar_arrive(smem_u32(&ctl.acc_empty[b]));
+                        else if (h == MT - 1) mbar_arrive(smem_u32(&ctl.acc_empty[b]));
+                        order = take_ticket(tile.split, rows32);
                     }
+                    order = __shfl_sync(0xffffffffu, order, 0);
+                    if (order != (unsigned)a.parts - 1u) continue;           // another part of these rows is still to come
+                    __threadfence();
+                    parts = base;
                 }
-                __syncwarp();
-                // whole rows out: w / 4 lanes per row
-                const int lpr = w / 4, rpi = 32 / lpr, sub = lane / lpr, lc = (lane - sub * lpr) * 4;
-                const int col = tile.n0 + c0 + lc;
-                const bool active = sub < rpi && col < a.n_cols;
-                float4 bias = make_float4(0.f, 0.f, 0.f, 0.f), sh = bias, t1 = bias, t2 = bias;
-                if (KIND == KIND_FPROP && a.bias && active) bias = ldg4(a.bias + col);
-                const bool stats = KIND == KIND_FPROP && a.stat_partial != nullptr;
-                const bool plain = KIND != KIND_FPROP || (!a.bias && a.act == AET_LINEAR);
-                float *out = a.out + col;
-                if (stats && active) sh = ldg4(a.stat_shift + col);
-                for (int r0 = 0; r0 < 32; r0 += 4 * rpi) {
-                    float4 o[4];
-                    int px[4];
+                for (int c0 = 0; c0 < a.bn; c0 += CHUNK) {
+                    const int w = a.bn - c0 < CHUNK ? a.bn - c0 : CHUNK;
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int r = r0 + u * rpi + sub;
-                        px[u] = __shfl_sync(0xffffffffu, pix, r & 31);
-                        if (r >= 32 || !active) px[u] = -1;
-                        o[u] = *reinterpret_cast<const float4 *>(mine + (r & 31) * PITCH + (active ? lc : 0));
+                    for (int h = 0; h < CHUNK; h += 32) {
+                        if (h >= w) break;
+                        const bool second = h + 16 < w;
+                        uint32_t v[32];
+                        if (split) {
+                            float f[32];
+#pragma unroll
+                            for (int q = 0; q < 32; ++q) f[q] = 0.f;
+                            // several parts' loads in flight: a trip takes a round to L2
+                            constexpr int FLY = X3 ? 2 : 4;
+                            for (int p = 0; p < a.parts; p += FLY) {
+                                float g[FLY][32];
+#pragma unroll
+                                for (int u = 0; u < FLY; ++u) {
+                                    const float *src = parts + (size_t)(p + u) * part_stride + (size_t)(c0 + h) * 32;
+#pragma unroll
+                                    for (int q = 0; q < 32; ++q)
+                                        g[u][q] = (p + u < a.parts && (q < 16 || second)) ? __ldcg(src + q * 32) : 0.f;
+                                }
+#pragma unroll
+                                for (int u = 0; u < FLY; ++u)
+#pragma unroll
+                                    for (int q = 0; q < 32; ++q) f[q] += g[u][q];
+                            }
+#pragma unroll
+                            for (int q = 0; q < 32; ++q) v[q] = __float_as_uint(f[q]);
+                        } else if (have) {
+                            const uint32_t src = acc + (uint32_t)(c0 + h);
+                            tmem_ld16_issue(src, v);
+                            if (second) tmem_ld16_issue(src + 16u, v + 16);
+                            tmem_ld_wait();
+                        } else {
+#pragma unroll
+                            for (int q = 0; q < 32; ++q) v[q] = 0u;
+                        }
+#pragma unroll
+                        for (int q = 0; q < 8; ++q)
+                            if (q < 4 || second)
+                                *reinterpret_cast<uint4 *>(mine + lane * PITCH + h + q * 4) = make_uint4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
                     }
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        if (!stats || px[u] < 0) continue;
-                        const float dx = o[u].x - sh.x, dy = o[u].y - sh.y, dz = o[u].z - sh.z, dw = o[u].w - sh.w;
-                        t1.x += dx; t1.y += dy; t1.z += dz; t1.w += dw;
-                        t2.x += dx * dx; t2.y += dy * dy; t2.z += dz * dz; t2.w += dw * dw;
-                    }
-                    if (!plain) {
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            o[u].x += bias.x; o[u].y += bias.y; o[u].z += bias.z; o[u].w += bias.w;
-                            o[u] = act_forward4(o[u], a.act);
+                    if (!split && h == MT - 1 && c0 + CHUNK >= a.bn) {   // the accumulator is read: the MMAs of the tile after the next may overwrite it
+                        tc_fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0) {
+                            if (PAIR) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl.acc_empty[b]), 0));
+                            else mbar_arrive(smem_u32(&ctl.acc_empty[b]));
                         }
                     }
+                    __syncwarp();
+                    // whole rows out: w / 4 lanes per row
+                    const int lpr = w / 4, rpi = 32 / lpr, sub = lane / lpr, lc = (lane - sub * lpr) * 4;
+                    const int col = tile.n0 + c0 + lc;
+                    const bool active = sub < rpi && col < a.n_cols;
+                    float4 bias = make_float4(0.f, 0.f, 0.f, 0.f), sh = bias, t1 = bias, t2 = bias;
+                    if (KIND == KIND_FPROP && a.bias && active) bias = ldg4(a.bias + col);
+                    const bool stats = KIND == KIND_FPROP && a.stat_partial != nullptr;
+                    const bool plain = KIND != KIND_FPROP || (!a.bias && a.act == AET_LINEAR);
+                    float *out = a.out + col;
+                    if (stats && active) sh = ldg4(a.stat_shift + col);
+                    for (int r0 = 0; r0 < 32; r0 += 4 * rpi) {
+                        float4 o[4];
+                        int px[4];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (px[u] >= 0) *reinterpret_cast<float4 *>(out + (size_t)px[u] * a.out_ld) = o[u];
-                }
-                if (stats) {   // the warp's row groups folded: one partial row per 32 rows of the GEMM
-                    float4 a1 = t1, a2 = t2;
-                    for (int k = 1; k < rpi; ++k) {
-                        const int src = lane + k * lpr;
-                        a1.x += __shfl_sync(0xffffffffu, t1.x, src); a1.y += __shfl_sync(0xffffffffu, t1.y, src);
-                        a1.z += __shfl_sync(0xffffffffu, t1.z, src); a1.w += __shfl_sync(0xffffffffu, t1.w, src);
-                        a2.x += __shfl_sync(0xffffffffu, t2.x, src); a2.y += __shfl_sync(0xffffffffu, t2.y, src);
-                        a2.z += __shfl_sync(0xffffffffu, t2.z, src); a2.w += __shfl_sync(0xffffffffu, t2.w, src);
+                        for (int u = 0; u < 4; ++u) {
+                            const int r = r0 + u * rpi + sub;
+                            px[u] = __shfl_sync(0xffffffffu, pix, r & 31);
+                            if (r >= 32 || !active) px[u] = -1;
+                            o[u] = *reinterpret_cast<const float4 *>(mine + (r & 31) * PITCH + (active ? lc : 0));
+                        }
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            if (!stats || px[u] < 0) continue;
+                            const float dx = o[u].x - sh.x, dy = o[u].y - sh.y, dz = o[u].z - sh.z, dw = o[u].w - sh.w;
+                            t1.x += dx; t1.y += dy; t1.z += dz; t1.w += dw;
+                            t2.x += dx * dx; t2.y += dy * dy; t2.z += dz * dz; t2.w += dw * dw;
+                        }
+                        if (!plain) {
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                o[u].x += bias.x; o[u].y += bias.y; o[u].z += bias.z; o[u].w += bias.w;
+                                o[u] = act_forward4(o[u], a.act);
+                            }
+                        }
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (px[u] >= 0) *reinterpret_cast<float4 *>(out + (size_t)px[u] * a.out_ld) = o[u];
                     }
-                    if (sub == 0 && active) {
-                        float *dst = a.stat_partial + (size_t)((tile.mg * (PAIR ? 2 : 1) + (int)prank) * 4 + warp) * 2 * a.out_ld + col;
-                        *reinterpret_cast<float4 *>(dst) = a1;
-                        *reinterpret_cast<float4 *>(dst + a.out_ld) = a2;
+                    if (stats) {   // the warp's row groups folded: one partial row per 32 rows of the GEMM
+                        float4 a1 = t1, a2 = t2;
+                        for (int k = 1; k < rpi; ++k) {
+                            const int src = lane + k * lpr;
+                            a1.x += __shfl_sync(0xffffffffu, t1.x, src); a1.y += __shfl_sync(0xffffffffu, t1.y, src);
+                            a1.z += __shfl_sync(0xffffffffu, t1.z, src); a1.w += __shfl_sync(0xffffffffu, t1.w, src);
+                            a2.x += __shfl_sync(0xffffffffu, t2.x, src); a2.y += __shfl_sync(0xffffffffu, t2.y, src);
+                            a2.z += __shfl_sync(0xffffffffu, t2.z, src); a2.w += __shfl_sync(0xffffffffu, t2.w, src);
+                        }
+                        if (sub == 0 && active) {
+                            float *dst = a.stat_partial + ((size_t)tile.mg * (ROWS / 32) + rows32) * 2 * a.out_ld + col;
+                            *reinterpret_cast<float4 *>(dst) = a1;
+                            *reinterpret_cast<float4 *>(dst + a.out_ld) = a2;
+                        }
                     }
+                    __syncwarp();
                 }
-                __syncwarp();
             }
         }
     } else if (warp == 4) {
@@ -368,7 +379,7 @@ conv_igemm_kernel(const __grid_constant__ IgemmMaps maps, const IgemmArgs a) {
             bool ok = true;
             for (int t = unit; t < total_tiles && ok; t += units, ++tcount) {
                 const IgemmTile tile = igemm_tile(a, t);
-                const uint32_t b = tcount & 1u, d = tmem + b * (uint32_t)a.bn;
+                const uint32_t b = tcount & 1u, d = tmem + b * MT * (uint32_t)a.bn;
                 if (!mbar_wait(smem_u32(&ctl.acc_empty[b]), ((tcount >> 1) & 1u) ^ 1u, abort_flag)) break;
                 tc_fence_after_sync();
                 uint32_t accumulate = 0;
@@ -394,7 +405,10 @@ conv_igemm_kernel(const __grid_constant__ IgemmMaps maps, const IgemmArgs a) {
                                 mma_tf32(d, ah, bh, idesc, 1u);
                             }
                         } else if (PAIR) mma_tf32_pair(d, ah, bh, idesc, jj > 0 ? 1u : accumulate);
-                        else mma_tf32(d, ah, bh, idesc, jj > 0 ? 1u : accumulate);
+                        else {
+                            mma_tf32(d, ah, bh, idesc, jj > 0 ? 1u : accumulate);
+                            if (MT > 1) mma_tf32(d + (uint32_t)a.bn, ah + ((BM * BK * 4) >> 4), bh, idesc, jj > 0 ? 1u : accumulate);
+                        }
                     }
                     accumulate = 1u;
                     if (PAIR) mma_commit_pair(empty0 + s * 8u, 3);
@@ -421,11 +435,15 @@ conv_igemm_kernel(const __grid_constant__ IgemmMaps maps, const IgemmArgs a) {
                 const IgemmTile tile = igemm_tile(a, t);
                 const IgemmClass &cl = a.cls[tile.cls];
                 const CUtensorMap *ma = &maps.a[tile.cls];
-                uint32_t m0 = (uint32_t)(tile.mt * (PAIR ? 256 : 128)) + prank * 128u;
-                if (m0 >= (uint32_t)cl.rows) m0 = 0;   // a pair's odd half past the end: any tile will do, it is not stored
-                const uint32_t n = fast_div(m0, cl.div_hw), rem = m0 - n * (uint32_t)cl.hw;
-                const uint32_t oh = fast_div(rem, cl.div_w), ow = rem - oh * (uint32_t)cl.w;
-                const int h0 = (int)oh * a.step + cl.h0, w0 = (int)ow * a.step + cl.w0;
+                int pn[MT], h0[MT], w0[MT];
+#pragma unroll
+                for (int h = 0; h < MT; ++h) {
+                    uint32_t m0 = (uint32_t)(tile.mt * ROWS) + (PAIR ? prank : (uint32_t)h) * 128u;
+                    if (m0 >= (uint32_t)cl.rows) m0 = 0;   // an odd half past the end: any tile will do, it is not stored
+                    const uint32_t n = fast_div(m0, cl.div_hw), rem = m0 - n * (uint32_t)cl.hw;
+                    const uint32_t oh = fast_div(rem, cl.div_w), ow = rem - oh * (uint32_t)cl.w;
+                    pn[h] = (int)n; h0[h] = (int)oh * a.step + cl.h0; w0[h] = (int)ow * a.step + cl.w0;
+                }
                 const int n0 = tile.n0 + (PAIR ? (int)prank * (a.bn / 2) : 0);
                 const int th = cl.th, tw = cl.tw, wtap0 = cl.r0 * a.S + cl.s0;
                 int tap = tile.slab0 / a.slabs_per_tap, cb = tile.slab0 - tap * a.slabs_per_tap;
@@ -440,8 +458,11 @@ conv_igemm_kernel(const __grid_constant__ IgemmMaps maps, const IgemmArgs a) {
                     for (int u = 0; u < here; ++u, sa += half_bytes) {
                         if (acts) {
                             const int oy = (KIND == KIND_FPROP ? tr : th - 1 - tr) * a.dil, ox = (KIND == KIND_FPROP ? ts : tw - 1 - ts) * a.dil;
-                            if (TO_LEADER) tma_load_im2col_pair(sa, ma, bar, cb * 32, w0, h0, (int)n, ox, oy);
-                            else tma_load_im2col(sa, ma, bar, cb * 32, w0, h0, (int)n, ox, oy);
+#pragma unroll
+                            for (int h = 0; h < MT; ++h) {
+                                if (TO_LEADER) tma_load_im2col_pair(sa, ma, bar, cb * 32, w0[h], h0[h], pn[h], ox, oy);
+                                else tma_load_im2col(sa + (uint32_t)h * (BM * BK * 4), ma, bar, cb * 32, w0[h], h0[h], pn[h], ox, oy);
+                            }
                         } else {
                             const uint32_t sb = sa + a_bytes;
                             const int wtap = wtap0 + a.tap_step * (tr * a.S + ts);
@@ -563,12 +584,14 @@ struct IgemmPlan {
     int bn;
     int splits;          // weight gradient: K splits of every tile
     int direct, parts;   // forward, data gradient: tiles computed whole, K parts of the others
+    int mt = 1;          // forward, data gradient: M tiles of a CTA
+    int rows() const { return BM * (pair ? 2 : mt); }
 };
-// Clocks of one K slab: its MMAs, or 100 and its bytes at 60 per clock.
+// Clocks of one K slab: its MMAs, or 100 and its bytes at 60 per clock (`mt`: M tiles of a CTA).
 // 3xTF32: three MMAs, and shared memory, which the low halves cross twice and the three MMAs read from, at 128 bytes per clock.
-double igemm_slab_clocks(int bn, bool pair, bool x3) {
-    const double mma = 4.0 * (bn <= 128 ? 70.0 : 70.0 + (bn - 128) * 62.0 / 128.0) * (x3 ? 3.0 : 1.0);
-    const double bytes = (128.0 + (pair ? bn / 2 : bn)) * 128.0;
+double igemm_slab_clocks(int bn, bool pair, bool x3, int mt = 1) {
+    const double mma = 4.0 * mt * (bn <= 128 ? 70.0 : 70.0 + (bn - 128) * 62.0 / 128.0) * (x3 ? 3.0 : 1.0);
+    const double bytes = (128.0 * mt + (pair ? bn / 2 : bn)) * 128.0;
     const double feed = x3 ? 200.0 + bytes * 6.0 / 128.0 : 100.0 + bytes / 60.0;
     return mma > feed ? mma : feed;
 }
@@ -579,51 +602,55 @@ IgemmPlan igemm_plan(const aet_context *ctx, const int *rows, int classes, int s
     IgemmPlan best = {false, 32, 1, 0, 1};
     double best_t = 1e30;
     const int full = round_up(n_cols, 32);
-    for (int pair = 0; pair < 2; ++pair)
-        for (int bn = 256; bn >= 32; bn -= 32) {
+    for (int mode = 0; mode < 3; ++mode) {   // single CTAs, pairs, single CTAs with two M tiles
+        const bool pair = mode == 1;
+        const int m = mode == 2 ? 2 : 1, tall = mode ? 256 : 128;
+        if (mode == 2 && x3) continue;
+        for (int bn = mode == 2 ? 128 : 256; bn >= 32; bn -= 32) {
             const int nt = (full + bn - 1) / bn;
             if (bn > full || (nt > 1 && bn < 64)) continue;
             if ((pair && bn % (2 * unit)) || (!pair && (bn % unit || (x3 && bn > 128)))) continue;
             int mt = 0;
-            for (int c = 0; c < classes; ++c) mt += (rows[c] + (pair ? 255 : 127)) / (pair ? 256 : 128);
+            for (int c = 0; c < classes; ++c) mt += (rows[c] + tall - 1) / tall;
             const int units = pair ? ctx->sm_count / 2 : ctx->sm_count, tiles = mt * nt, rem = tiles % units;
-            const double tile = slabs * igemm_slab_clocks(bn, pair != 0, x3) + 400.0 + bn * 4.0;
-            const double base = (double)(tiles / units) * tile + 3000.0 + bn * 12.0 + (pair ? 1200.0 : 0.0);
+            const double slab = igemm_slab_clocks(bn, pair, x3, m), tile = slabs * slab + 400.0 + bn * 4.0 * m;
+            const double base = (double)(tiles / units) * tile + 3000.0 + bn * 12.0 * m + (pair ? 1200.0 : 0.0);
             double t = base + (rem ? tile : 0.0);
-            if (t < best_t * 0.999) { best_t = t; best = {pair != 0, bn, 1, tiles, 1}; }
+            if (t < best_t * 0.999) { best_t = t; best = {pair, bn, 1, tiles, 1, m}; }
             if (!rem || !ctx->opt[OPT_FD_SPLIT]) continue;
             for (int parts = 2; parts <= 8 && rem * parts <= units && slabs / parts >= 6; ++parts) {
-                t = base + (slabs + parts - 1) / parts * igemm_slab_clocks(bn, pair != 0, x3) + 400.0 + bn * 8.0 + 1500.0 + parts * bn * (x3 ? 12.0 : 6.0);
-                if (t < best_t * 0.999) { best_t = t; best = {pair != 0, bn, 1, tiles - rem, parts}; }
+                t = base + (slabs + parts - 1) / parts * slab + 400.0 + bn * 8.0 * m + 1500.0 + parts * bn * (x3 ? 12.0 : 6.0 * m);
+                if (t < best_t * 0.999) { best_t = t; best = {pair, bn, 1, tiles - rem, parts, m}; }
             }
         }
+    }
     return best;
 }
 
-// "i2c_", p(air) or n(o pair), filters (or channels) of a tile
+// "i2c_", p(air) or n(o pair), filters (or channels) of a tile, x2: two M tiles
 void igemm_label(char *variant, size_t size, const IgemmPlan &plan, bool x3) {
-    snprintf(variant, size, "i2c_%s%d%s", plan.pair ? "p" : "n", plan.bn, x3 ? "_x3" : "");
+    snprintf(variant, size, "i2c_%s%d%s", plan.pair ? "p" : "n", plan.bn, x3 ? "_x3" : (plan.mt > 1 ? "x2" : ""));
 }
 
-template <int KIND, bool PAIR, bool X3>
+template <int KIND, bool PAIR, bool X3, int MT = 1>
 int igemm_launch(aet_context *ctx, const IgemmMaps &maps, IgemmArgs &a, const char *name, const char *variant, double flops) {
     const int bnc = PAIR ? a.bn / 2 : a.bn;
     a.b_bytes = (uint32_t)bnc * BK * 4;
-    a.tx_bytes = (uint32_t)BM * BK * 4 + a.b_bytes;
-    const size_t stage = (size_t)a.tx_bytes * 2, staging = (size_t)BM * ((X3 ? 32 : IG_CHUNK) + 4) * 4;
+    a.tx_bytes = (uint32_t)MT * BM * BK * 4 + a.b_bytes;
+    const size_t stage = (size_t)a.tx_bytes * (MT > 1 ? 1 : 2), staging = (size_t)BM * ((X3 ? 32 : IG_CHUNK) + 4) * 4;
     int stages = (int)((219 * 1024 - 1024 - staging) / stage);
     if (stages > IG_MAX_STAGES) stages = IG_MAX_STAGES;
     a.stages = stages;
-    a.tmem_cols = pow2_cols(2 * a.bn);
+    a.tmem_cols = pow2_cols(2 * MT * a.bn);
     a.status = ctx->status_dev;
     const size_t smem_bytes = stage * stages + staging + 1024;
-    AET_TRY(ctx_smem_attr(ctx, conv_igemm_kernel<KIND, PAIR, X3>));
+    AET_TRY(ctx_smem_attr(ctx, conv_igemm_kernel<KIND, PAIR, X3, MT>));
     const int tiles = a.direct_tiles + (a.m_tiles * a.n_tiles - a.direct_tiles) * a.parts, units = PAIR ? ctx->sm_count / 2 : ctx->sm_count;
     const int grid = (tiles < units ? tiles : units) * (PAIR ? 2 : 1);
     LaunchScope scope(ctx, name, 0, flops, variant);
     a.span = ctx->span_ptr;
-    if (PAIR) launch_k_cluster(ctx->stream, dim3(grid), dim3(224 + (X3 ? IG_CONVERTERS * 32 : 0)), smem_bytes, 2, 1, conv_igemm_kernel<KIND, PAIR, X3>, maps, a);
-    else launch_k(ctx->stream, dim3(grid), dim3(224 + (X3 ? IG_CONVERTERS * 32 : 0)), smem_bytes, conv_igemm_kernel<KIND, PAIR, X3>, maps, a);
+    if (PAIR) launch_k_cluster(ctx->stream, dim3(grid), dim3(224 + (X3 ? IG_CONVERTERS * 32 : 0)), smem_bytes, 2, 1, conv_igemm_kernel<KIND, PAIR, X3, MT>, maps, a);
+    else launch_k(ctx->stream, dim3(grid), dim3(224 + (X3 ? IG_CONVERTERS * 32 : 0)), smem_bytes, conv_igemm_kernel<KIND, PAIR, X3, MT>, maps, a);
     return aet_check_launch(name);
 }
 
@@ -637,15 +664,16 @@ int igemm_run(aet_layer *l, const ConvArgs &ca, const IgemmPlan &plan, const Ige
     if (plan.parts > 1) {
         // the batch statistics' partial rows (already handed out at the arena's start) stay in front of the parts
         const size_t split_tiles = (size_t)a.m_tiles * a.n_tiles - plan.direct;
-        if (split_tiles * (plan.pair ? 8 : 4) > (size_t)kTickets) { aet_set_error("convolution: more split tiles than tickets"); return AET_E_INVALID; }
+        if (split_tiles * (plan.rows() / 32) > (size_t)kTickets) { aet_set_error("convolution: more split tiles than tickets"); return AET_E_INVALID; }
         const size_t stats = ca.stats ? ca.stats->floats : 0;
         float *arena = nullptr;
-        AET_TRY(ctx_scratch(ctx, (stats + split_tiles * plan.parts * plan.bn * BM * (plan.pair ? 2 : 1)) * sizeof(float), &arena));
+        AET_TRY(ctx_scratch(ctx, (stats + split_tiles * plan.parts * plan.bn * plan.rows()) * sizeof(float), &arena));
         if (ca.stats) ca.stats->partial = a.stat_partial = arena;
         a.partial = arena + stats;
         a.tickets = ctx->tickets + (ctx->on_side ? kTickets : 0);
     }
     if (x3) return plan.pair ? igemm_launch<KIND, true, true>(ctx, maps, a, name, variant, flops) : igemm_launch<KIND, false, true>(ctx, maps, a, name, variant, flops);
+    if (plan.mt > 1) return igemm_launch<KIND, false, false, 2>(ctx, maps, a, name, variant, flops);
     return plan.pair ? igemm_launch<KIND, true, false>(ctx, maps, a, name, variant, flops) : igemm_launch<KIND, false, false>(ctx, maps, a, name, variant, flops);
 }
 
@@ -686,11 +714,11 @@ int igemm_fprop(aet_layer *l, const ConvArgs &a, double flops) {
     IgemmClass &c = t.cls[0];
     c.hw = g.OH * g.OW; c.w = g.OW; c.div_hw = make_fastdiv(c.hw); c.div_w = make_fastdiv(c.w);
     c.rows = a.n_rows; c.h0 = c.w0 = -p; c.th = g.R; c.tw = g.S;
-    c.tile_end = t.m_tiles = (a.n_rows + (plan.pair ? 255 : 127)) / (plan.pair ? 256 : 128);
+    c.tile_end = t.m_tiles = (a.n_rows + plan.rows() - 1) / plan.rows();
     t.classes = 1; t.out = a.out; t.bias = a.bias; t.act = a.act; t.stat_shift = a.stat_shift; t.stat_partial = a.stat_partial;
     t.bn = plan.bn; t.n_cols = a.n_cols; t.out_ld = a.out_ld; t.step = g.sx; t.tap_step = 1; t.dil = g.dil; t.S = g.S;
     t.slabs_per_tap = slabs_per_tap; t.n_tiles = (a.n_cols + plan.bn - 1) / plan.bn;
-    if (a.stat_rows_out) *a.stat_rows_out = t.m_tiles * (plan.pair ? 8 : 4);
+    if (a.stat_rows_out) *a.stat_rows_out = t.m_tiles * (plan.rows() / 32);
     return igemm_run<KIND_FPROP>(l, a, plan, maps, t, "conv_fprop_tma", flops);
 }
 
@@ -734,7 +762,7 @@ int igemm_dgrad(aet_layer *l, const ConvArgs &a, double flops) {
     const int bnc = plan.pair ? plan.bn / 2 : plan.bn;
     for (int k = 0; k < t.classes; ++k) {
         AET_TRY(get_map_im2col(l, 22 + k, a.src_a, g.kp, g.ys, g.OW, g.OH, g.N, box[k], false, &maps.a[k]));
-        t.m_tiles += (rows[k] + (plan.pair ? 255 : 127)) / (plan.pair ? 256 : 128);
+        t.m_tiles += (rows[k] + plan.rows() - 1) / plan.rows();
         t.cls[k].tile_end = t.m_tiles;
     }
     {

@@ -252,3 +252,48 @@ def test_conv_of_few_images_shares_k_in_clusters(aet, ctx, oracle, shape):
         ctx.profile(0)
     assert {"conv_fprop_tma.cl", "conv_dgrad_tma.cl"} <= names, names
     check(got, ref, TOL_TF32)
+
+
+@pytest.mark.parametrize("shape,names_of", [
+    ((43, 96, 27, 27, 64, 5, 1, 2, 2), ("fprop_tma.i2c_n64x2", "dgrad_tma.i2c_n96x2")),     # the last tile's second half is empty
+    ((40, 64, 40, 40, 96, 3, 2, 1, 0), ("dgrad_tma.i2c_n64x2",)),                           # four residue classes, each with such a tile
+    ((52, 48, 41, 41, 40, 3, 1, 1, 1), ("fprop_tma.i2c_n64x2", "dgrad_tma.i2c_n64x2")),     # last round split along K, ragged channels
+])
+def test_two_pixel_tiles_per_cta(aet, ctx, oracle, shape, names_of):
+    ctx.set_math(aet.MATH_TF32)
+    ctx.profile(1)
+    try:
+        got, ref = conv_case(aet, ctx, oracle, *shape, seed=960 + shape[1], threads=True)
+        names = variants_used(ctx)
+    finally:
+        ctx.profile(0)
+    check(got, ref, TOL_TF32)
+    for want in names_of:
+        assert any(n.startswith("conv_" + want) for n in names), (want, names)
+
+
+def test_batch_statistics_of_two_pixel_tiles_per_cta(aet, ctx):
+    """The statistics that come out of such tiles' epilogue, by way of the output they normalise: against the gather kernel."""
+    n, c, h, k = 43, 96, 27, 60
+    rng = np.random.default_rng(5)
+    x = rng.standard_normal((n, c, h, h)).astype(np.float32)
+    w = rng.standard_normal((k, c, 5, 5)).astype(np.float32) * 0.03
+    out = {}
+    for gather in (0, 1):
+        ctx.set_option("gather_only", gather)
+        try:
+            layer = aet.ConvolutionalLayer(ctx, n, h, h, c, k, 5, 1, 1, 2, aet.LINEAR, 1, 1)
+            xin = aet.Tensor(ctx, n, c, h, h)
+            xin.write(x)
+            layer.write(aet.P_WEIGHTS, w)
+            ctx.profile(1)
+            layer.forward(aet.make_state(input=xin, train=1))
+            assert gather or any(v.startswith("conv_fprop_tma.i2c_n64x2") for v in variants_used(ctx))
+            out[gather] = layer.read(aet.P_OUTPUT), layer.read(aet.P_ROLLING_MEAN), layer.read(aet.P_ROLLING_VARIANCE)
+            layer.close()
+            xin.close()
+        finally:
+            ctx.profile(0)
+            ctx.set_option("gather_only", 0)
+    for a, b in zip(out[0], out[1]):
+        assert np.isfinite(a).all() and rel_l2(a, b) <= TOL_TF32
