@@ -37,24 +37,30 @@ bool s2d_geom(const aet_layer *l, S2dGeom *out) {
     return true;
 }
 
-// regrouped input: one thread per 16-byte cell of xb, cells of one block pixel consecutive
-__global__ void __launch_bounds__(256) s2d_input_kernel(const float *__restrict__ x, float *__restrict__ xb, int N, int H, int W, int pad,
-                                                        int s, int hb, int wb, int cpad, long long total) {
+// regrouped input: four 16-byte cells of xb per thread, all loaded before the first is stored, cells of one block pixel
+// consecutive; bound by memory once the divisions are multiplications (128 images of 227x227, 211 MB: 47 -> 33 us, 6.4 TB/s)
+constexpr int S2D_CELLS = 4;
+struct S2dDivs {
+    FastDiv per, wb, hb, s;
+};
+__global__ void __launch_bounds__(256) s2d_input_kernel(const float *__restrict__ x, float *__restrict__ xb, int H, int W, int pad, int s,
+                                                        int hb, int wb, int per, S2dDivs div, unsigned total) {
     pdl_enter();
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    const int per = cpad / 4;
-    const int cell = (int)(i % per);
-    long long q = i / per;
-    const int bx = (int)(q % wb); q /= wb;
-    const int by = (int)(q % hb);
-    const int n = (int)(q / hb);
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (cell < s * s) {
-        const int iy = by * s + cell / s - pad, ix = bx * s + cell % s - pad;
-        if (iy >= 0 && iy < H && ix >= 0 && ix < W) v = ldg4(x + ((size_t)((size_t)n * H + iy) * W + ix) * 4);
+    const unsigned i0 = blockIdx.x * (256u * S2D_CELLS) + threadIdx.x;
+    float4 v[S2D_CELLS];
+#pragma unroll
+    for (int u = 0; u < S2D_CELLS; ++u) {
+        const unsigned i = i0 + u * 256u;
+        v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i >= total) continue;
+        const unsigned q = fast_div(i, div.per), row = fast_div(q, div.wb), n = fast_div(row, div.hb);
+        const int cell = (int)(i - q * (unsigned)per), bx = (int)(q - row * (unsigned)wb), by = (int)(row - n * (unsigned)hb);
+        const int dy = (int)fast_div((unsigned)cell, div.s), iy = by * s + dy - pad, ix = bx * s + cell - dy * s - pad;
+        if (dy < s && (unsigned)iy < (unsigned)H && (unsigned)ix < (unsigned)W) v[u] = ldg4(x + ((size_t)((size_t)n * H + iy) * W + ix) * 4);
     }
-    *reinterpret_cast<float4 *>(xb + (size_t)i * 4) = v;
+#pragma unroll
+    for (int u = 0; u < S2D_CELLS; ++u)
+        if (i0 + u * 256u < total) *reinterpret_cast<float4 *>(xb + (size_t)(i0 + u * 256u) * 4) = v[u];
 }
 
 // regrouped filter: wb[k][ry][rx][cell] = w[k][ry*s + dy][rx*s + dx] (16 bytes = the 4 padded channels of a tap)
@@ -131,8 +137,10 @@ int s2d_regroup_input(aet_layer *l, const S2dGeom &g, const float *x) {
     aet_context *ctx = l->ctx;
     const long long total = (long long)l->batch * g.hb * g.wb * (g.cpad / 4);
     LaunchScope scope(ctx, "conv_s2d_input", (double)l->batch * l->h * l->w * 16.0 + (double)total * 16.0, 0);
-    launch_k(ctx->stream, (unsigned)((total + 255) / 256), 256, 0, s2d_input_kernel, x, l->s2d_x, l->batch, l->h, l->w, l->pad, g.s, g.hb,
-             g.wb, g.cpad, total);
+    const S2dDivs div = {make_fastdiv((uint32_t)(g.cpad / 4)), make_fastdiv((uint32_t)g.wb), make_fastdiv((uint32_t)g.hb), make_fastdiv((uint32_t)g.s)};
+    const int per_block = 256 * S2D_CELLS;   // fewer than 2^29 cells in all (see s2d_geom)
+    launch_k(ctx->stream, (unsigned)((total + per_block - 1) / per_block), 256, 0, s2d_input_kernel, x, l->s2d_x, l->h, l->w, l->pad, g.s, g.hb,
+             g.wb, g.cpad / 4, div, (unsigned)total);
     return aet_check_launch("conv_s2d_input");
 }
 
