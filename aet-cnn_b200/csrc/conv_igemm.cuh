@@ -11,9 +11,9 @@
 // 128 x 128 x 32 slab of TF32 brings 32 KB for 308 clocks of MMA.  So tiles are as large as the problem fills the chip with: a CTA pair
 // (cta_group::2) computes 256 pixels x up to 256 filters, each CTA fetching its own 128 pixels and half of the filters.
 // Where there are 128 columns or less, a CTA by itself does better with two M tiles (MT = 2) for one set of filters: 96 filters
-// bring 22 KB a tile and slab instead of 28, which a pair's 22 KB do not match (pairs get 47 bytes per clock where lone CTAs, whose
-// equal filters meet on the way, get 60).  5x5 taps, 256 -> 96 channels on 27x27, batch 128: 258 -> 230 us (as pairs 277); 3x3,
-// 48 -> 96 on 57x57: 125 -> 117; 96 filters at batch 50: 52 -> 46.
+// bring 22 KB a tile and slab instead of 28.  A pair brings 22 KB as well, but was slower than either: 5x5 taps, 256 -> 96
+// channels on 27x27, batch 128: 258 us alone, 277 as pairs, 230 with two M tiles; 3x3, 64 -> 96 on 57x57: 125 as pairs, 117;
+// the same at batch 50: 52, 46.
 // CTAs are persistent and hold two accumulators in TMEM: the epilogue of a tile (four warps) runs under the main loop
 // of the next.  The tiles of an incomplete last round are split along K over the chip and summed by the last to finish.
 //
