@@ -1230,20 +1230,20 @@ __device__ __forceinline__ void linhead_cost(const LinHeadArgs &a, int n, int wa
     }
 }
 
-__global__ void __launch_bounds__(256) linhead_forward_kernel(const LinHeadArgs a) {
-    pdl_enter();
-    extern __shared__ float xs[];           // cp pooled inputs, then 32 logits
-    const int n = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// Pooled inputs of sample n (xs, kept in xbar for the weight gradient) and behind them its logits, in the order of additions that
+// training steps and calls one by one share: pixels in turn, a lane's channels in turn, then the lanes.  FLY: pixels in flight.
+template <int FLY>
+__device__ __forceinline__ void linhead_logits(const LinHeadArgs &a, int n, int warp, int lane, float *xs) {
     const float *xn = a.x + (size_t)n * a.S * a.cp;
     for (int c = threadIdx.x; c < a.cp; c += 256) {
         float s = 0.f;
         int px = 0;
-        for (; px + 8 <= a.S; px += 8) {   // eight loads in flight; the sum keeps the pixel order
-            float t[8];
+        for (; px + FLY <= a.S; px += FLY) {
+            float t[FLY];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) t[u] = xn[(size_t)(px + u) * a.cp + c];
+            for (int u = 0; u < FLY; ++u) t[u] = xn[(size_t)(px + u) * a.cp + c];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) s += t[u];
+            for (int u = 0; u < FLY; ++u) s += t[u];
         }
         for (; px < a.S; ++px) s += xn[(size_t)px * a.cp + c];
         s /= a.S;
@@ -1260,74 +1260,33 @@ __global__ void __launch_bounds__(256) linhead_forward_kernel(const LinHeadArgs 
         if (lane == 0) lg[k] = d + a.b[k];
     }
     __syncthreads();
+}
+
+__global__ void __launch_bounds__(256) linhead_forward_kernel(const LinHeadArgs a) {
+    pdl_enter();
+    extern __shared__ float xs[];           // cp pooled inputs, then 32 logits
+    const int n = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    linhead_logits<8>(a, n, warp, lane, xs);
     float err = 0.f, d;
-    if (warp == 0) err = linhead_softmax(a, n, lane, lane < a.classes ? lg[lane] : 0.f, d);
+    if (warp == 0) err = linhead_softmax(a, n, lane, lane < a.classes ? xs[a.cp + lane] : 0.f, d);
     linhead_cost(a, n, warp, lane, err);
 }
 
 // In a training step, whose backward pass comes next, the block goes on to the delta of the pooled layer (`pd`), for which it has
-// everything at hand.  A chain of latencies, a block per sample: a thread's weights are asked for with its pixels, and every
-// class' sum over the channels is folded at the end (as fast at 128 samples; a prediction of one image, 0.5 us slower this way,
-// keeps the kernel above).  The layer below no longer waits for a kernel that forms the delta and the weight gradient; what is
-// left of that one, off the chain now, runs beside the rest: sixteen steps of the 32x32 classifier at batch 128 3.75 -> 3.70 ms.
+// everything at hand.  A chain of latencies, a block per sample: the weights come to L1 while the pixels are on their way.  The
+// layer below no longer waits for a kernel that forms the delta and the weight gradient; what is left of that one, off the
+// chain now, runs beside the rest: sixteen steps of the 32x32 classifier at batch 128 3.75 -> 3.70 ms.
 __global__ void __launch_bounds__(256) linhead_step_kernel(const LinHeadArgs a) {
     pdl_enter();
-    __shared__ float part[8][32], g[32];
+    extern __shared__ float xs[];           // as above
+    __shared__ float g[32];
     const int n = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const float *xn = a.x + (size_t)n * a.S * a.cp;
-    float acc[32];
-#pragma unroll
-    for (int k = 0; k < 32; ++k) acc[k] = 0.f;
-    for (int c = threadIdx.x; c < a.cp; c += 256) {
-        float w[32];
-#pragma unroll
-        for (int k = 0; k < 32; ++k) {
-            if (k >= a.classes) break;
-            w[k] = a.w[(size_t)k * a.cp + c];
-        }
-        float s = 0.f;
-        int px = 0;
-        for (; px + 16 <= a.S; px += 16) {   // sixteen loads in flight; the sum keeps the pixel order
-            float t[16];
-#pragma unroll
-            for (int u = 0; u < 16; ++u) t[u] = xn[(size_t)(px + u) * a.cp + c];
-#pragma unroll
-            for (int u = 0; u < 16; ++u) s += t[u];
-        }
-        for (; px + 4 <= a.S; px += 4) {
-            float t[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) t[u] = xn[(size_t)(px + u) * a.cp + c];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) s += t[u];
-        }
-        for (; px < a.S; ++px) s += xn[(size_t)px * a.cp + c];
-        s /= a.S;
-        a.xbar[(size_t)n * a.cp + c] = s;
-#pragma unroll
-        for (int k = 0; k < 32; ++k) {
-            if (k >= a.classes) break;
-            acc[k] += w[k] * s;
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 32; ++k) {
-        if (k >= a.classes) break;
-        float d = acc[k];
-#pragma unroll
-        for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-        if (lane == 0) part[warp][k] = d;
-    }
-    __syncthreads();
+    for (int i = threadIdx.x * 32; i < a.classes * a.cp; i += 256 * 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(a.w + i));
+    linhead_logits<16>(a, n, warp, lane, xs);
     float err = 0.f;
     if (warp == 0) {
-        float v = 0.f, d;
-        if (lane < a.classes) {
-#pragma unroll
-            for (int q = 0; q < 8; ++q) v += part[q][lane];
-            v += a.b[lane];
-        }
-        err = linhead_softmax(a, n, lane, v, d);
+        float d;
+        err = linhead_softmax(a, n, lane, lane < a.classes ? xs[a.cp + lane] : 0.f, d);
         g[lane] = a.loss_scale * d;
     }
     __syncthreads();
@@ -2373,8 +2332,7 @@ int k_linhead_forward(aet_layer *conv, aet_layer *avg, aet_layer *sm, const floa
     LinHeadArgs h = make_linhead(conv, avg, sm, x, truth, pd);
     LaunchScope s(ctx, "linear_head_forward", (pd ? 8.0 : 4.0) * h.N * h.S * h.cp + 4.0 * h.classes * h.cp, (pd ? 4.0 : 2.0) * h.N * h.classes * h.cp,
                   pd ? "dx" : nullptr);
-    if (pd) launch_k(ctx->stream, h.N, 256, 0, linhead_step_kernel, h);
-    else launch_k(ctx->stream, h.N, 256, (size_t)(h.cp + 32) * sizeof(float), linhead_forward_kernel, h);
+    launch_k(ctx->stream, h.N, 256, (size_t)(h.cp + 32) * sizeof(float), pd ? linhead_step_kernel : linhead_forward_kernel, h);
     return aet_check_launch("linear_head_forward");
 }
 // `pd` null: the forward pass has formed that delta, the weight and bias gradients are left

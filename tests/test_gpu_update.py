@@ -117,17 +117,23 @@ def compare_all(aet, fused, plain, tol):
 @pytest.mark.parametrize("case", [(37, 32, 3, 64, 128, 10, "mtcs"), (5, 24, 1, 128, 96, 3, "cpu"), (9, 36, 2, 61, 260, 32, "mtcs")])
 @pytest.mark.parametrize("graph", [False, True])
 def test_head_delta_with_the_forward_pass(aet, ctx, case, graph):
-    """In a training step the classifier head forms its input's delta with the forward pass.  The same numbers are added up in
-    the same order as call by call; what the compiler contracts differently in the two forms is a rounding of a delta."""
+    """In a training step the classifier head forms its input's delta with the forward pass.  Every sum of the head has the order that
+    it has call by call: outputs, deltas and the head's parameters are the same bit for bit.  (The other layers' weight gradients
+    may be split otherwise in a step, where they overwrite the gradient instead of adding to it.)"""
     batch, side, channels, n0, n1, classes, parity = case
     text = IMAGE_NET % (batch, side, side, channels, parity, n0, n1, classes)
     fused, plain = two_nets(aet, ctx, text, batch)
     try:
         fused.use_graph(graph)
         ctx.profile(0 if graph else 1)
-        for _ in range(2):
+        for step in range(2):
             fused.train_device()
             step_by_calls(aet, plain)
+            if step == 0:
+                for i in range(fused.layer_count):
+                    a, b = fused.layer(i), plain.layer(i)
+                    for which in (aet.P_OUTPUT, aet.P_DELTA) + ((aet.P_WEIGHTS, aet.P_WEIGHT_UPDATES, aet.P_BIASES, aet.P_BIAS_UPDATES) if i == 4 else ()):
+                        assert not a.param_count(which) or np.array_equal(a.read(which), b.read(which)), (i, which)
         if not graph:
             names = variants_used(ctx)
             assert any(n.startswith("linear_head_forward.dx") for n in names), names
