@@ -445,7 +445,10 @@ extern "C" int aet_layer_forward(aet_layer *l, aet_state state) {
             cv->lin_fwd_pending = false;
             if (l->head_avg->head_forward_pending && state.input == l->head_avg->output) {
                 l->head_avg->head_forward_pending = false;
-                aet_tensor *pd = truth && l->ctx->step_forward && l->net && cv->index > 0 ? l->net->layers[cv->index - 1]->delta : nullptr;
+                // In a training step the backward pass follows, and where the softmax is the last layer nothing else writes to its
+                // delta or to the one in front of the head in between: the latter comes with the forward pass.
+                const bool ahead = truth && l->ctx->step_forward && l->net && l->index + 1 == (int)l->net->layers.size() && cv->index > 0;
+                aet_tensor *pd = ahead ? l->net->layers[cv->index - 1]->delta : nullptr;
                 AET_TRY(k_linhead_forward(cv, l->head_avg, l, cv->lin_input->d, truth, pd ? pd->d : nullptr));
                 cv->lin_dx_done = pd != nullptr;
                 cv->lin_used = truth != nullptr;

@@ -147,6 +147,28 @@ def test_head_delta_with_the_forward_pass(aet, ctx, case, graph):
         plain.close()
 
 
+@pytest.mark.parametrize("behind", ["[softmax]\n", "[dropout]\nprobability=0.5\n\n[softmax]\n", "[shortcut]\nfrom=-2\nactivation=linear\n\n[softmax]\n",
+                                    "[shortcut]\nfrom=-4\nactivation=linear\n\n[softmax]\n"])
+def test_layers_behind_the_classifier_head(aet, ctx, behind):
+    """What the layers behind a head's softmax add to its delta, or to that of the layer in front of the head, counts in a
+    training step as it does call by call."""
+    text = (HEAD % (9, 16, 16, 3) + CONV % (32, 3, 1, "leaky", "") + "[maxpool]\nsize=16\nstride=16\npadding=0\n\n" + CONV % (10, 1, 0, "leaky", "") +
+            CONV % (10, 1, 0, "linear", "") + "[avgpool]\n\n[softmax]\n\n" + behind)
+    fused, plain = two_nets(aet, ctx, text, 9)
+    try:
+        if "dropout" in behind:
+            r = np.random.default_rng(7).random(fused.layer(6).param_count(aet.P_RAND), np.float32)
+            for n in (fused, plain):
+                n.layer(6).write(aet.P_RAND, r)
+        for _ in range(2):
+            fused.train_device()
+            step_by_calls(aet, plain)
+        compare_all(aet, fused, plain, 3.3e-5)   # as above
+    finally:
+        fused.close()
+        plain.close()
+
+
 @pytest.mark.parametrize("case", [(3, 3, 2, "leaky", 0, 27, 96), (2, 2, 2, "relu", 0, 16, 20), (3, 3, 2, "linear", 0, 14, 33), (2, 2, 2, "leaky", 1, 15, 32),
                                   (3, 3, 2, "tanh", 0, 13, 32)])
 @pytest.mark.parametrize("dropout", [False, True])
