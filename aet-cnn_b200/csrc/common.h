@@ -33,6 +33,7 @@ void aet_set_error(const char *fmt, ...);
     do {                                                                                            \
         cudaError_t e__ = (call);                                                                   \
         if (e__ != cudaSuccess) {                                                                   \
+            cudaGetLastError();   /* reported here: not the next launch's error as well */          \
             aet_set_error("%s failed: %s (%s:%d)", #call, cudaGetErrorString(e__), __FILE__, __LINE__); \
             return AET_E_CUDA;                                                                      \
         }                                                                                           \

@@ -1,4 +1,5 @@
 """Helpers shared by the GPU parity tests: run one layer through the C ABI and through the oracle."""
+import contextlib
 import os
 from concurrent.futures import ThreadPoolExecutor
 
@@ -95,3 +96,15 @@ def kernels_used(ctx):
 def variants_used(ctx):
     """Full labels ("kernel.variant") of the profiled launches: which code path each launcher picked."""
     return {r["name"] for r in ctx.profile_read()}
+
+
+@contextlib.contextmanager
+def device_memory_taken(leave):
+    """All but `leave` bytes of the device's free memory belong to somebody else for a while: allocations beyond that fail."""
+    import torch
+    taken = torch.empty(torch.cuda.mem_get_info()[0] - leave, dtype=torch.uint8, device="cuda")
+    try:
+        yield
+    finally:
+        del taken
+        torch.cuda.empty_cache()

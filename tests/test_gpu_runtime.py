@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 from conftest import rel_l2
+from gpu_util import device_memory_taken
 from oracle import binding as ob
 from oracle import cfgfile
 
@@ -295,3 +296,33 @@ def test_option_switches(aet, ctx):
     ctx.set_option("rows", 1)
     with pytest.raises(aet.AetError):
         ctx.set_option("no_such_switch", 1)
+
+
+def test_a_failed_allocation_is_the_failing_call_s_error_alone(aet):
+    """A backward pass that finds no memory for its scratch is refused; with the memory there, the next calls work."""
+    rng = np.random.default_rng(3)
+    n, c, h, k = 32, 512, 8, 512
+    x, w, dy = [rng.standard_normal(s).astype(np.float32) for s in ((n, c, h, h), (k, c, 3, 3), (n, k, h, h))]
+    got = []
+    for short in (False, True):   # the first round also loads the kernels, which takes device memory of its own
+        own = aet.Context(0)
+        layer, xin, dx = aet.ConvolutionalLayer(own, n, h, h, c, k, 3, 1, 1, 1, aet.LEAKY, 0, 1), aet.Tensor(own, n, c, h, h), aet.Tensor(own, n, c, h, h)
+        layer.write(aet.P_WEIGHTS, w)
+        xin.write(x)
+        st = aet.make_state(input=xin, delta=dx, train=1)
+        layer.forward(st)
+        layer.write(aet.P_DELTA, dy)
+        own.synchronize()
+        if short:
+            with device_memory_taken(10 << 20):
+                with pytest.raises(aet.AetError, match="out of memory"):
+                    layer.backward(st)
+            layer.forward(st)
+            layer.write(aet.P_DELTA, dy)
+            layer.update(n, 0.0, 0.0, 0.0)   # clears what the refused pass has added to the bias gradient
+        layer.backward(st)
+        got.append((layer.read(aet.P_OUTPUT), dx.read(), layer.read(aet.P_WEIGHT_UPDATES), layer.read(aet.P_BIAS_UPDATES)))
+        for thing in (layer, xin, dx, own):
+            thing.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
