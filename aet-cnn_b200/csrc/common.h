@@ -130,7 +130,7 @@ struct aet_context {
     bool wgrad_fresh = false;     // set by a training step without subdivisions: the gradient arena is zero when backward starts, the weight gradients may overwrite
     bool step_forward = false;          // a training step's forward pass, whose backward pass is queued right behind it
     bool in_step = false;               // a training step's backward pass, right behind its forward pass
-    aet_network *update_in = nullptr;   // set by a training step whose update follows at once: weight gradients may apply it themselves
+    aet_network *update_in = nullptr;   // set by a training step whose update follows at once: weight gradients may be left to it
     bool on_side = false, side_pending = false;
     float *scratch_side = nullptr;
     size_t scratch_side_bytes = 0;
@@ -205,7 +205,8 @@ struct aet_layer {
     ParamArena own_arena;
     ParamSegment seg_w, seg_b, seg_s;
     int seg_id = 0;                      // of the weights, in the network's update tables
-    bool updated = false;                // this pass's weight gradient has applied the update to the weights already
+    bool updated = false;                // this pass's weight gradient is formed by a kernel that applies the update to the weights
+    bool update_pending = false;         // ... which is still to be queued
     float *mean = nullptr, *variance = nullptr, *rolling_mean = nullptr, *rolling_variance = nullptr;
     float *inv_std = nullptr;            // per-channel 1/std in the parity mode's form
     float *bwd_coef = nullptr;           // [3][ocp] coefficients of the BN backward apply pass
@@ -550,10 +551,11 @@ struct ConvStats {
 int conv_fprop(aet_layer *l, const float *x, float *y, const float *bias, int act_in_epilogue, ConvStats *stats = nullptr);
 int conv_dgrad(aet_layer *l, const float *dy, float *dx);
 int conv_wgrad(aet_layer *l, const float *x, const float *dy, float *dw, int accumulate);
-// The weight gradient can apply the step's update in its epilogue (then it has to run behind the data gradient, which reads
-// the weights); conv_wgrad_update runs it and marks the layer as updated.
+// The weight gradient can apply the step's update in its epilogue; conv_pending_updates queues it for all layers that wait for it.
+// It has to run behind the layer's data gradient, which reads the weights, and where the pass runs as it is queued behind all
+// that can still be refused: an error leaves the weights as they were.
 bool conv_update_ok(const aet_layer *l);
-int conv_wgrad_update(aet_layer *l, const float *x, const float *dy);
+int conv_pending_updates(aet_network *net);
 void conv_release(aet_layer *l);
 
 int k_bn_stats(aet_layer *l, int update_rolling, const ConvStats *from_epilogue = nullptr);

@@ -941,10 +941,23 @@ bool conv_update_ok(const aet_layer *l) {
     return updated < kMaxUpdated && igemm_update_ok(l, layer_geom(l));
 }
 
-int conv_wgrad_update(aet_layer *l, const float *x, const float *dy) {
-    const ConvGeom g = layer_geom(l);
-    AET_TRY(igemm_wgrad_update(l, g, x, dy, 2.0 * g.N * (double)g.K * g.C));
-    l->updated = true;
+int conv_pending_updates(aet_network *net) {
+    aet_layer *layers[kMaxUpdated];
+    IgemmUpdate plans[kMaxUpdated];
+    int n = 0;
+    for (size_t i = net->layers.size(); i-- > 0;) {   // what can be refused is done for all of them before the first is queued
+        aet_layer *l = net->layers[i];
+        if (!l->update_pending) continue;
+        const aet_tensor *x = i ? net->layers[i - 1]->output : net->input;
+        AET_TRY(igemm_update_setup(l, layer_geom(l), x->d, l->delta->d, plans[n]));
+        layers[n++] = l;
+        l->update_pending = false;
+    }
+    for (int k = 0; k < n; ++k) {
+        const ConvGeom g = layer_geom(layers[k]);
+        net->ctx->prof_tag = layers[k]->index;
+        AET_TRY(igemm_update_run(net->ctx, plans[k], 2.0 * g.N * (double)g.K * g.C));
+    }
     return AET_OK;
 }
 

@@ -513,8 +513,13 @@ bool igemm_update_ok(const aet_layer *l, const ConvGeom &g) {
     return l->ctx->math == AET_MATH_TF32 && l->groups == 1 && g.OH == 1 && g.OW == 1 && g.R == 1 && g.S == 1 && g.N <= 8 * BK &&
            (double)g.K * g.cp >= 1048576.0 && (double)g.K * g.cp < 1073741824.0 && igemm_wgrad_ok(l, g, box);
 }
-int igemm_wgrad_update(aet_layer *l, const ConvGeom &g, const float *x, const float *dy, double flops) {
-    aet_context *ctx = l->ctx;
+struct IgemmUpdate {
+    IgemmWgradArgs args;
+    CUtensorMap x;
+    const CUtensorMap *dy;
+};
+int igemm_update_setup(aet_layer *l, const ConvGeom &g, const float *x, const float *dy, IgemmUpdate &up) {
+    const aet_context *ctx = l->ctx;
     Im2colBox box;
     if (!igemm_wgrad_ok(l, g, box)) { aet_set_error("internal: layer cannot update itself"); return AET_E_INVALID; }
     // tiles of the width whose last round wastes least (a tile's cost: its columns, and 16 for its start)
@@ -525,15 +530,15 @@ int igemm_wgrad_update(aet_layer *l, const ConvGeom &g, const float *x, const fl
         const int rounds = (mt * ((g.K + bn - 1) / bn) + ctx->sm_count - 1) / ctx->sm_count;
         if (rounds * (bn + 16) < best) { best = rounds * (bn + 16); plan.bn = bn; }
     }
-    IgemmWgradArgs t = {};
-    CUtensorMap mx;
-    const CUtensorMap *mdy;
-    AET_TRY(igemm_wgrad_setup(l, g, x, dy, box, plan, t, &mx, &mdy));
-    const aet_network *net = ctx->update_in;
-    t.W = layer_W(l); t.U = layer_U(l); t.seg = net->seg_table + 4 * l->seg_id; t.hyper = net->hyper_dev;
+    up.args = {};
+    AET_TRY(igemm_wgrad_setup(l, g, x, dy, box, plan, up.args, &up.x, &up.dy));
+    up.args.W = layer_W(l); up.args.U = layer_U(l); up.args.seg = l->net->seg_table + 4 * l->seg_id; up.args.hyper = l->net->hyper_dev;
+    return AET_OK;
+}
+int igemm_update_run(aet_context *ctx, IgemmUpdate &up, double flops) {
     char variant[32];
-    snprintf(variant, sizeof(variant), "i2c_n%d_sgd", plan.bn);
-    return igemm_wgrad_launch<false, false, true>(ctx, mx, *mdy, t, variant, flops);
+    snprintf(variant, sizeof(variant), "i2c_n%d_sgd", up.args.bn);
+    return igemm_wgrad_launch<false, false, true>(ctx, up.x, *up.dy, up.args, variant, flops);
 }
 
 }  // namespace

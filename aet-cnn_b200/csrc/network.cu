@@ -356,7 +356,11 @@ int net_backward(aet_network *net, aet_state state, bool exchange = true) {
         if (net->xchg_active && pend_hi - pend_lo <= net->xchg_cap) { net->tail_lo = pend_lo; net->tail_n = pend_hi - pend_lo; }
         else AET_TRY(issue_allreduce(net, pend_lo, pend_hi, slot++));
     }
-    AET_TRY(side_join(ctx));
+    // behind the last data gradient, beside the weight gradients that are still running
+    int r = conv_pending_updates(net);
+    if (r == AET_OK) r = side_join(ctx);
+    else side_join(ctx);
+    AET_TRY(r);
     if (dp && slot > 0) {
         // Option "comm_stamps": one-thread kernels read %globaltimer before and after the wait for the collectives, and
         // the second adds the difference to a running sum - how long the main stream sat idle for communication.
@@ -388,13 +392,20 @@ int run_step(aet_network *net, bool final) {
     if (net->ctx->wgrad_fresh && final && !net->adam && !net->comm && !net->xchg_active) net->ctx->update_in = net;
     net->ctx->in_step = true;
     const int br = net_backward(net, st, final);
+    const bool fresh = net->ctx->wgrad_fresh;
     net->ctx->in_step = false;
     net->ctx->wgrad_fresh = false;
     net->ctx->update_in = nullptr;
-    if (br != AET_OK)
-        for (aet_layer *l : net->layers) l->updated = false;
-    AET_TRY(br);
     net->grad_clean = false;
+    if (br != AET_OK) {
+        for (aet_layer *l : net->layers) l->updated = l->update_pending = false;
+        // The parameters are as they were; so is the arena, which was zero before this pass, once it is cleared of what the pass
+        // has queued.  (A pass that was being captured has not run.  With other ranks attached, collectives may still use it.)
+        if (fresh && !net->comm && !net->xchg_active)
+            net->grad_clean = net->ctx->capturing ||
+                              cudaMemsetAsync(net->arena.G, 0, net->arena.used * sizeof(float), net->ctx->stream) == cudaSuccess;
+        return br;
+    }
     if (!final) return AET_OK;   // gradients keep accumulating in the arena until the group's last call
     net->ctx->prof_tag = -1;   // the update belongs to no single layer
     if (net->n_blocks) AET_TRY(net->adam ? k_adam_arena(net) : k_sgd_arena(net));

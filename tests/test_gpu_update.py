@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from conftest import rel_l2
-from gpu_util import variants_used
+from gpu_util import device_memory_taken, variants_used
 
 pytestmark = pytest.mark.gpu
 
@@ -95,6 +95,43 @@ def test_self_updating_layers_scrub_and_hold_still(aet, ctx):
         finally:
             fused.close()
             plain.close()
+
+
+def parameters(aet, net):
+    return [net.layer(i).read(which) for i in range(net.layer_count) for which in (aet.P_WEIGHTS, aet.P_WEIGHT_UPDATES, aet.P_BIASES, aet.P_BIAS_UPDATES)
+            if net.layer(i).param_count(which)]
+
+
+def test_a_step_that_fails_leaves_everything_as_it_was(aet):
+    """No memory for a convolution's weight gradient, after the fully connected layers behind it had theirs: no parameter has
+    moved, no gradient is left over, and the step that is made again is the step."""
+    text = (HEAD % (32, 8, 8, 16) + CONV % (512, 3, 1, "leaky", "") + CONV % (512, 3, 1, "leaky", "") + CONV % (256, 8, 0, "relu", "") +
+            CONV % (10, 1, 0, "linear", "") + "[softmax]\n")
+    own = aet.Context(0)
+    failing, other = two_nets(aet, own, text, 32)
+    warm, spare = two_nets(aet, own, text, 32)
+    try:
+        # the kernels are loaded and the main stream has its scratch; the second stream's is still to come
+        own.set_option("overlap_wgrad", 0)
+        own.profile(1)
+        warm.train_device()
+        assert any("_sgd" in n for n in variants_used(own)), variants_used(own)
+        own.profile(0)
+        own.set_option("overlap_wgrad", 1)
+        before = parameters(aet, failing)
+        with device_memory_taken(10 << 20):
+            with pytest.raises(aet.AetError, match="out of memory"):
+                failing.train_device()
+        for a, b in zip(before, parameters(aet, failing)):
+            assert np.array_equal(a, b)
+        for _ in range(2):
+            failing.train_device()
+            other.train_device()
+            for a, b in zip(parameters(aet, failing), parameters(aet, other)):
+                assert np.array_equal(a, b)
+    finally:
+        for thing in (failing, other, warm, spare, own):
+            thing.close()
 
 
 IMAGE_NET = ("[net]\nbatch=%d\nwidth=%d\nheight=%d\nchannels=%d\nparity=%s\nlearning_rate=0.01\nmomentum=0.9\ndecay=0.0005\npolicy=constant\n\n"
