@@ -506,12 +506,17 @@ int igemm_wgrad(aet_layer *l, const ConvArgs &ca, float *dw, int accumulate, dou
 // weights, from a batch that is a few K slabs, is bound by memory: written, read again and cleared by the update it costs
 // 28 bytes per weight (4096 x 9216 at batch 128: 100 us alone and 157 of the update's 255), in the epilogue the 16 that the
 // weights and their momentum take (16 warps with eight rows each in flight 124 us, 5.3 TB/s; 12 warps with sixteen rows asked
-// for after the products 164; eight steps of the 227x227 network 18.33 -> 17.55 -> 17.22 ms).  From a million weights on and up to
-// 8 slabs (256 images); below that, or where K is longer, the launch and the products count.  Offsets are 32 bits of bytes.
+// for after the products 164; eight steps of the 227x227 network 18.33 -> 17.55 -> 17.22 ms).
+// From six million weights on: below that few tiles and one kernel behind the other cost more than the traffic.  A step of three fully
+// connected layers, gradient and update apart -> together, us, at 64 and 256 images: 1024 x 1024 72 -> 74, 78 -> 82; 2048 x 2048
+// 84 -> 82, 93 -> 96; 4096 x 1000 84 -> 84, 98 -> 98; 3072 x 2048 95 -> 92, 119 -> 107; 4096 x 2048 114 -> 100, 139 -> 123;
+// 4096 x 4096 176 -> 146, 214 -> 183.  Of the larger ones two or three lose 2 to 3 % at 8 images (2048 x 4096 115 -> 118), the
+// others gain 10 to 20 %.  Up to 8 slabs (256 images): where K is longer the gain shrinks (4096 x 4096 at 1024 images 332 -> 318) and
+// one accumulator would have to sum it all.  Offsets are 32 bits of bytes.
 bool igemm_update_ok(const aet_layer *l, const ConvGeom &g) {
     Im2colBox box;
     return l->ctx->math == AET_MATH_TF32 && l->groups == 1 && g.OH == 1 && g.OW == 1 && g.R == 1 && g.S == 1 && g.N <= 8 * BK &&
-           (double)g.K * g.cp >= 1048576.0 && (double)g.K * g.cp < 1073741824.0 && igemm_wgrad_ok(l, g, box);
+           (double)g.K * g.cp >= 6.0 * 1048576.0 && (double)g.K * g.cp < 1073741824.0 && igemm_wgrad_ok(l, g, box);
 }
 struct IgemmUpdate {
     IgemmWgradArgs args;
