@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 from conftest import rel_l2
+from gpu_util import variants_used
 from oracle import binding as ob
 
 pytestmark = pytest.mark.gpu
@@ -104,6 +105,28 @@ def test_maxpool_values_and_indices_bit_exact(aet, ctx, oracle, mode, geom):
     assert np.array_equal(idx, io), "argmax indices must be bit-exact"
     assert np.array_equal(y, yo)
     assert np.allclose(got_pd, oracle.maxpool_backward(dy, io, prev0), rtol=1e-6, atol=1e-6)
+
+
+@pytest.mark.parametrize("size", [2, 3, 4])
+def test_maxpool_of_large_maps_runs_from_the_end(aet, ctx, size):
+    """Above 72 MB the blocks run from the end of the map.  Values and indices are those of the same images in two smaller calls."""
+    n, c, h = 283, 63, 32
+    x = np.random.default_rng(size).standard_normal((n, c, h, h)).astype(np.float32)
+    got = []
+    for part in (x, x[:180], x[180:]):
+        layer, xin = aet.MaxPoolLayer(ctx, len(part), h, h, c, size, 2, 2, 0, 1), aet.Tensor(ctx, *part.shape)
+        xin.write(part)
+        ctx.profile(1)
+        layer.forward(aet.make_state(input=xin, train=1))
+        assert ("maxpool_fwd.end" in variants_used(ctx)) == (len(part) == n)
+        ctx.profile(0)
+        image = c * h * h   # indices count from the first image of a call
+        got.append((layer.read(aet.P_OUTPUT), layer.read(aet.P_INDEXES) + (180 * image if len(got) == 2 else 0)))
+        layer.close()
+        xin.close()
+    for whole, first, second in zip(*got):
+        assert np.array_equal(whole, np.concatenate([first, second]))
+
 
 
 def test_avgpool_forward_backward(aet, ctx, oracle):
