@@ -1,6 +1,4 @@
 """Training steps whose weight gradients apply the update in their epilogue, against the same step made call by call."""
-import os
-
 import numpy as np
 import pytest
 
@@ -17,7 +15,7 @@ def two_nets(aet, ctx, text, batch):
     rng = np.random.default_rng(batch)
     nets = [aet.NNetwork(ctx, cfg_text=text, train=1, batch=batch) for _ in range(2)]
     x = rng.random(nets[0].input_shape, np.float32)
-    t = np.eye(nets[0].outputs, dtype=np.float32)[rng.integers(0, nets[0].outputs, batch)]
+    t = np.eye(nets[0].outputs, dtype=np.float32)[rng.integers(0, nets[0].outputs, nets[0].batch)]
     for n in nets:
         n.use_graph(False)
         n.input.write(x)
@@ -76,35 +74,150 @@ def test_fully_connected_layers_update_themselves(aet, ctx, shape, graph):
         plain.close()
 
 
-def test_self_updating_layers_scrub_and_hold_still(aet, ctx):
-    """Non-finite pending updates are cleared as by the update kernel, and a layer that is not updated yet only collects."""
-    for extra in ("", "dont_update=1\n"):
-        text = HEAD % (16, 8, 8, 32) + CONV % (64, 3, 1, "leaky", "") + CONV % (1540, 8, 0, "relu", extra) + CONV % (10, 1, 0, "linear", "") + "[softmax]\n"
-        fused, plain = two_nets(aet, ctx, text, 16)
-        try:
+def self_updates(ctx):
+    return sum(r["launches"] for r in ctx.profile_read() if "_sgd" in r["name"])
+
+
+WIDE = HEAD % (32, 1, 1, 2512) + CONV % (2512, 1, 0, "relu", "") + CONV % (10, 1, 0, "linear", "") + "[softmax]\n"   # 6.3 million weights
+
+
+def test_a_captured_step_lets_its_layers_update_themselves(aet, ctx):
+    """Such a layer's gradient is never in the arena: a mark there is still there after the step.  The separate kernels write the
+    gradient over it and the update clears it."""
+    import ctypes
+    import torch
+    torch.cuda.init()
+    cudart = ctypes.CDLL("libcudart.so.12")
+    net, spare = two_nets(aet, ctx, WIDE, 32)
+    try:
+        arena, count = net.grad_arena()
+        mark, seen = ctypes.c_float(7.0), ctypes.c_float(0.0)
+        middle = ctypes.c_void_p(arena + 4 * (count // 2))   # the wide layer takes nearly all of the arena
+
+        def copy(dst, src, kind):
+            ctx.synchronize()
+            assert cudart.cudaMemcpy(dst, src, ctypes.c_size_t(4), ctypes.c_int(kind)) == 0
+
+        net.use_graph(True)
+        for expected in (7.0, 7.0, 0.0):
+            for _ in range(3):
+                net.train_device()
+            copy(middle, ctypes.byref(mark), 1)
+            if expected == 0.0:   # a backward pass by hand: the arena no longer counts as empty
+                net.backward(aet.make_state(input=net.input, truth=net.truth, train=1))
+            net.train_device()
+            copy(ctypes.byref(seen), middle, 2)
+            assert seen.value == expected
+            copy(middle, ctypes.byref(ctypes.c_float(0.0)), 1)
+    finally:
+        net.close()
+        spare.close()
+
+
+@pytest.mark.parametrize("guard", ["adam", "subdivisions", "3xtf32", "batch", "small", "communicator", "left over"])
+def test_layers_that_must_not_update_themselves(aet, ctx, guard):
+    """Where somebody else has a part in the gradient or the update, or the rule's range ends, the separate kernels run."""
+    batch, text = 32, WIDE
+    if guard == "adam":
+        text = WIDE.replace("policy=constant", "policy=constant\nadam=1")
+    if guard == "batch":
+        batch = 257
+    if guard == "small":
+        text = WIDE.replace("filters=2512", "filters=2400")
+    if guard == "subdivisions":
+        batch, text = 0, WIDE.replace("batch=32", "batch=64\nsubdivisions=2")
+    if guard == "3xtf32":
+        ctx.set_math(aet.MATH_3XTF32)
+    net, plain = two_nets(aet, ctx, text, batch)
+    try:
+        if guard == "communicator":
+            net.comm_init(aet.comm_unique_id(), 0, 1)
+        if guard == "left over":
+            state = aet.make_state(input=net.input, truth=net.truth, train=1)
+            for n in (net, plain):
+                n.forward(state)
+                n.backward(state)
+        ctx.profile(1)
+        for _ in range(2 if guard == "subdivisions" else 1):
+            net.train_device()
+        assert self_updates(ctx) == 0, variants_used(ctx)
+        ctx.profile(0)
+        if guard == "adam":   # divides by the gradient's size: the rounding of one that is nearly zero becomes a whole step
+            return
+        if guard == "subdivisions":
+            state = aet.make_state(input=plain.input, truth=plain.truth, train=1)
+            plain.forward(state)
+            plain.backward(state)
+        step_by_calls(aet, plain)
+        compare(aet, net, plain, 2e-5)
+    finally:
+        ctx.profile(0)
+        ctx.set_math(aet.MATH_TF32)
+        net.close()
+        plain.close()
+
+
+def test_a_ninth_wide_layer_is_updated_with_the_others(aet, ctx):
+    text = HEAD % (16, 1, 1, 2512) + 9 * (CONV % (2512, 1, 0, "leaky", "")) + CONV % (10, 1, 0, "linear", "") + "[softmax]\n"
+    fused, plain = two_nets(aet, ctx, text, 16)
+    try:
+        ctx.profile(1)
+        fused.train_device()
+        assert self_updates(ctx) == 8, variants_used(ctx)
+        ctx.profile(0)
+        step_by_calls(aet, plain)
+        compare(aet, fused, plain, 2e-5)
+    finally:
+        ctx.profile(0)
+        fused.close()
+        plain.close()
+
+
+# 4096 x 1540: the last eight filters of the last tile are four
+@pytest.mark.parametrize("held", [False, True])
+def test_self_updating_layers_scrub_and_hold_still(aet, ctx, held):
+    """Non-finite weights and pending updates are replaced as by the update kernel, and a layer that is not updated yet collects
+    its gradient, unscaled.  (The other side has a communicator of one rank: the same training step with the separate kernels.)"""
+    text = (HEAD % (16, 8, 8, 32) + CONV % (64, 3, 1, "leaky", "") + CONV % (1540, 8, 0, "relu", "dont_update=1\n" if held else "") + CONV % (10, 1, 0, "linear", "") +
+            "[softmax]\n")
+    fused, plain = two_nets(aet, ctx, text, 16)
+    try:
+        plain.comm_init(aet.comm_unique_id(), 0, 1)
+        spots = [(0, 0, 0), (700, 5, 63), (1539, 63, 17)]   # filter, tap, channel: the first, a later tile's, one of the last four filters'
+        host = [k * 4096 + c * 64 + tap for k, tap, c in spots]
+        device = [k * 4096 + tap * 64 + c for k, tap, c in spots]
+        if not held:
             for n in (fused, plain):
-                u = n.layer(1).read(aet.P_WEIGHT_UPDATES)
+                w, u = n.layer(1).read(aet.P_WEIGHTS), n.layer(1).read(aet.P_WEIGHT_UPDATES)
+                w[host] = np.nan, np.inf, -np.inf
                 u[[3, 1017, len(u) - 1]] = np.nan, np.inf, -np.inf
-                if not extra:
-                    n.layer(1).write(aet.P_WEIGHT_UPDATES, u)
-            start = fused.layer(1).read(aet.P_WEIGHTS)
-            for step in range(2):
-                fused.train_device()
-                if not extra and step == 0:
-                    with pytest.raises(aet.AetError):
-                        ctx.check()
-                if extra:   # iteration 1: held
-                    assert np.array_equal(fused.layer(1).read(aet.P_WEIGHTS), start) == (step == 0)
-                    continue
-                step_by_calls(aet, plain)
-                if step == 0:
-                    with pytest.raises(aet.AetError):
-                        ctx.check()
-            if not extra:
-                compare(aet, fused, plain, 2e-5)
-        finally:
-            fused.close()
-            plain.close()
+                n.layer(1).write(aet.P_WEIGHTS, w)
+                n.layer(1).write(aet.P_WEIGHT_UPDATES, u)
+        start = fused.layer(1).read(aet.P_WEIGHTS)
+        ctx.profile(1)
+        for step in range(2):
+            fused.train_device()
+            assert self_updates(ctx) == step + 1
+            if not held and step == 0:
+                with pytest.raises(aet.AetError):
+                    ctx.check()
+            plain.train_device()
+            assert self_updates(ctx) == step + 1
+            if not held and step == 0:
+                with pytest.raises(aet.AetError):
+                    ctx.check()
+            w, u = [[n.layer(1).read(which) for n in (fused, plain)] for which in (aet.P_WEIGHTS, aet.P_WEIGHT_UPDATES)]
+            assert np.isfinite(w[0]).all() and np.isfinite(u[0]).all()
+            assert rel_l2(*w) <= 2e-5 and rel_l2(*u) <= 2e-5
+            if held:   # iteration 1: held, and the gradient is there
+                assert np.array_equal(w[0], start) == (step == 0) and np.abs(u[0]).max() > 0
+            elif step == 0:   # 1 / (index + 1), and then the step: the rate times the decay of it
+                assert np.allclose(w[0][host], 1.0 / (np.array(device) + 1.0), rtol=2 * 0.05 * 0.0005)
+            copy_parameters(aet, fused, plain)
+    finally:
+        ctx.profile(0)
+        fused.close()
+        plain.close()
 
 
 def parameters(aet, net):
