@@ -604,7 +604,9 @@ void pinned_block_give(void *block);
 int k_param_hash(aet_context *ctx, const float *p, size_t count, uint64_t *hash_dev);
 int k_augment(aet_context *ctx, const float *src_nchw, int n, int c, int sh, int sw, float *dst_nhwc, int size, int cp,
               const aet_augment *params_dev);
-constexpr int kMaxUpdated = 8;   // most layers of a network that update themselves in one pass
+// most layers of a network that update themselves in one pass: their blocks travel in the update kernel's arguments, which every
+// block of it searches, and from the ninth layer on the separate kernels are there anyway
+constexpr int kMaxUpdated = 8;
 constexpr int kTopkLanes = 32;   // lists of up to this many entries are held by a warp's lanes
 int k_top_k(aet_context *ctx, const float *scores, int samples, int n, int ld, int k, int *index_dev, StatusTap tap = {});
 

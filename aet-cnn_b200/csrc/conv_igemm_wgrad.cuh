@@ -510,9 +510,8 @@ int igemm_wgrad(aet_layer *l, const ConvArgs &ca, float *dw, int accumulate, dou
 // From six million weights on: below that few tiles and one kernel behind the other cost more than the traffic.  A step of three fully
 // connected layers, gradient and update apart -> together, us, at 64 and 256 images: 1024 x 1024 72 -> 74, 78 -> 82; 2048 x 2048
 // 84 -> 82, 93 -> 96; 4096 x 1000 84 -> 84, 98 -> 98; 3072 x 2048 95 -> 92, 119 -> 107; 4096 x 2048 114 -> 100, 139 -> 123;
-// 4096 x 4096 176 -> 146, 214 -> 183.  Of the larger ones two or three lose 2 to 3 % at 8 images (2048 x 4096 115 -> 118), the
-// others gain 10 to 20 %.  Up to 8 slabs (256 images): where K is longer the gain shrinks (4096 x 4096 at 1024 images 332 -> 318) and
-// one accumulator would have to sum it all.  Offsets are 32 bits of bytes.
+// 4096 x 4096 176 -> 146, 214 -> 183.  Up to 8 slabs (256 images): where K is longer the gain shrinks (4096 x 4096 at 1024 images
+// 332 -> 318) and one accumulator would have to sum it all.  Offsets are 32 bits of bytes.
 bool igemm_update_ok(const aet_layer *l, const ConvGeom &g) {
     Im2colBox box;
     return l->ctx->math == AET_MATH_TF32 && l->groups == 1 && g.OH == 1 && g.OW == 1 && g.R == 1 && g.S == 1 && g.N <= 8 * BK &&
