@@ -7,12 +7,13 @@
 // copy brings 128 consecutive OUTPUT positions of one filter tap and 32 channels, across row and image ends and with the
 // convolution's stride, so every tile is full and one thread feeds the pipeline whatever the geometry.
 //
-// What bounds it is the L2 -> SM path (52 to 60 bytes per clock and SM with all of them pulling), then the tensor pipe: a
-// 128 x 128 x 32 slab of TF32 brings 32 KB for 308 clocks of MMA.  So tiles are as large as the problem fills the chip with: a CTA pair
-// (cta_group::2) computes 256 pixels x up to 256 filters, each CTA fetching its own 128 pixels and half of the filters.
-// Where there are 128 columns or less, a CTA by itself does better with two M tiles (MT = 2) for one set of filters: 96 filters
-// bring 22 KB a tile and slab instead of 28.  A pair brings 22 KB as well, but was slower than either: 5x5 taps, 256 -> 96
-// channels on 27x27, batch 128: 258 us alone, 277 as pairs, 230 with two M tiles; 3x3, 64 -> 96 on 57x57: 125 as pairs, 117;
+// Larger tiles are faster per product, so they are as large as the problem fills the chip with: a CTA pair (cta_group::2) computes
+// 256 pixels x up to 256 filters, each CTA fetching its own 128 pixels and half of the filters (700 TFLOP/s; lone 128 x 96 tiles
+// 440).  A slab of 128 x 128 x 32 brings 32 KB for 308 clocks of MMA and L2 delivers 52 to 60 bytes per clock and SM with all of them
+// pulling, but neither those bytes nor the SM clock alone set the pace: one activation tile for all taps of a filter row (45 %
+// fewer bytes) was no faster, and a slab takes the same 455 ns at 1.6 and at 1.95 GHz.
+// Where there are 128 columns or less, a CTA by itself can take two M tiles (MT = 2) for one set of filters.  5x5 taps, 256 -> 96
+// channels on 27x27, batch 128: 258 us with one, 277 as pairs, 230 with two; 3x3, 64 -> 96 on 57x57: 125 as pairs, 117;
 // the same at batch 50: 52, 46.
 // CTAs are persistent and hold two accumulators in TMEM: the epilogue of a tile (four warps) runs under the main loop
 // of the next.  The tiles of an incomplete last round are split along K over the chip and summed by the last to finish.
@@ -587,8 +588,9 @@ struct IgemmPlan {
     int mt = 1;          // forward, data gradient: M tiles of a CTA
     int rows() const { return BM * (pair ? 2 : mt); }
 };
-// Clocks of one K slab: its MMAs, or 100 and its bytes at 60 per clock (`mt`: M tiles of a CTA).
-// 3xTF32: three MMAs, and shared memory, which the low halves cross twice and the three MMAs read from, at 128 bytes per clock.
+// Clocks of one K slab, as a fit to measured layers and not a claim of what bounds them: its MMAs, or 100 and its bytes at 60 per
+// clock (`mt`: M tiles of a CTA).  3xTF32: three MMAs, or 200 and six times its bytes at 128 per clock.  Whole kernels take 1.3 to
+// 1.4 times the sums of this model in the median, whichever tile they use; it is there to choose between tiles.
 double igemm_slab_clocks(int bn, bool pair, bool x3, int mt = 1) {
     const double mma = 4.0 * mt * (bn <= 128 ? 70.0 : 70.0 + (bn - 128) * 62.0 / 128.0) * (x3 ? 3.0 : 1.0);
     const double bytes = (128.0 * mt + (pair ? bn / 2 : bn)) * 128.0;

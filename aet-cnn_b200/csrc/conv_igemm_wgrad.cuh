@@ -8,9 +8,13 @@
 // layers waste nothing.  With the filters along N, a TMEM lane is an input channel, so a warp stores 128 contiguous
 // bytes of the [filter][tap][channel] gradient per register and the epilogue needs no shared memory.
 //
-// As in the forward kernel the L2 -> SM path bounds it, so pairs of CTAs compute 256 x 256 tiles; K is split over the grid to
+// As in the forward kernel larger tiles are faster, so pairs of CTAs compute 256 x 256; K is split over the grid to
 // fill whole rounds, partial gradients are summed in a fixed order by the reduce kernel.  One split that may overwrite
-// stores straight into the gradient.
+// stores straight into the gradient.  In TF32 two groups of four epilogue warps share a tile's filters.
+//
+// UPDATE: the fully connected layers of a training step.  Sixteen epilogue warps add the products to the momenta, move the
+// weights and write no gradient at all.  The layer's data gradient reads the old weights: it has to be queued first, on the stream
+// that this kernel's stream waits for.
 #pragma once
 
 namespace {

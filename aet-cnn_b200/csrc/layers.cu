@@ -497,10 +497,11 @@ extern "C" int aet_layer_backward(aet_layer *l, aet_state state) {
     case AET_CONVOLUTIONAL: {
         AET_TRY(check_input(l, state.input));
         if (l->lin_bwd_pending) {
-            // fused linear head: softmax and avg-pool backward, this layer's data, weight and bias gradients in one kernel
+            // fused linear head: softmax and avg-pool backward, this layer's data, weight and bias gradients in one kernel.
+            // Where the forward pass has formed the deltas already, the weight and bias gradients are left, which only the
+            // update waits for.
             l->lin_bwd_pending = false;
             if (!pd) return fail_invalid("linear head backward needs the previous layer's delta");
-            // what is left of a delta that came with the forward pass is for the update alone
             const bool ahead = l->lin_dx_done;
             l->lin_dx_done = false;
             if (ahead && l->ctx->overlap_wgrad) AET_TRY(side_begin(l->ctx));
